@@ -1,7 +1,7 @@
 // Factor-solve of one band system with no device allocation (included once, by strut_cuda.cu).
 //
 // strut_gpu_band_solve_noalloc runs the BandGeneral / BandSPD factor and solve of the Newton
-// kernel (band_lu_smem / band_chol_smem and the same substitutions) on one system the caller
+// kernel (band_lu_cta, band_lu_smem, band_chol_smem and the same substitutions) on one system the caller
 // already holds in device memory.  The dense partial-pivot fallback of BandGeneral
 // (linear_solver_backend.mojo:175-240, 650-657) needs an n x n work matrix and n pivots; here
 // they live in file-scope static device arrays sized for kNoAllocMaxN, whose device addresses
@@ -34,6 +34,8 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
     extern __shared__ __align__(16) double smem_one[];
     __shared__ double red[32];
     __shared__ int red_r[32];
+    __shared__ double s_rk[2], s_z[2];  // band_lu_cta
+    __shared__ int s_flag[2];
     const int tid = threadIdx.x, nt = blockDim.x;
     const int rw = 2 * bw + 1;
     double* Kb = smem_one;
@@ -41,20 +43,31 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
     double* w = R + n;
     double* xs = w + n;
     double* fac = xs + n;
-    for (int t = tid; t < n * rw; t += nt) {
-        const int i = t / rw, j = i + t % rw - bw;
-        double v = 0.0;
-        if (j >= 0 && j < n) {
-            if (!spd)
-                v = band[t];
-            else if (j <= i)
-                v = band[(size_t)i * (bw + 1) + (i - j)];
+    // (the slots of columns outside the matrix are never used)
+    if (!spd) {
+#pragma unroll 8
+        for (int t = tid; t < n * rw; t += nt) Kb[t] = band[t];
+    } else {
+#pragma unroll 4
+        for (int t = tid; t < n * (bw + 1); t += nt) {
+            const int i = t / (bw + 1);
+            Kb[i * rw + bw - (t - i * (bw + 1))] = band[t];
         }
-        Kb[t] = v;
     }
     for (int i = tid; i < n; i += nt) R[i] = rhs[i];
     __syncthreads();
-    int rc = spd ? band_chol_smem(Kb, n, bw, rw, fac) : band_lu_smem(Kb, n, bw, rw, fac);
+    bool forward = false;  // w holds L^-1 rhs already
+    int rc;
+    if (spd) {
+        rc = band_chol_smem(Kb, n, bw, rw, fac);
+    } else if (bw <= kLuRowsMax) {
+        for (int i = tid; i < n; i += nt) w[i] = R[i];
+        __syncthreads();
+        rc = band_lu_cta<false>(Kb, n, bw, rw, (int)(w - Kb), s_rk, s_z, s_flag);
+        forward = true;
+    } else {
+        rc = band_lu_smem(Kb, n, bw, rw, fac);
+    }
     bool use_dense = false;
     if (rc == 6) {
         // the whole n x n work matrix is rewritten from the caller's band before the dense LU
@@ -77,9 +90,9 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
         if (use_dense)
             dense_solve_warp(dense, piv, n, R, w, xs);
         else if (spd)
-            band_solve_chol_warp(Kb, n, bw, rw, R, w, xs);
+            band_solve_chol_warp(Kb, n, bw, rw, R, w, xs, fac);
         else
-            band_solve_lu_warp(Kb, n, bw, rw, R, w, xs);
+            band_solve_lu_warp(Kb, n, bw, rw, forward ? nullptr : R, w, xs, fac);
     }
     __syncthreads();
     for (int i = tid; i < n; i += nt) x[i] = xs[i];

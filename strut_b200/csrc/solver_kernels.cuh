@@ -18,6 +18,7 @@
 //   tests                     nonlinear_convergence.mojo:8-20, transient_nonlinear.mojo:2798-2811
 #pragma once
 
+#include "band_warp.cuh"
 #include "kernels.cuh"
 
 namespace strut {
@@ -122,7 +123,7 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 }
 
 // Right-looking band LU without pivoting (Doolittle, unit-lower multipliers stored in place)
-// on the n x (2bw+1) band in shared memory.  Step k computes the multiplier a_ik / a_kk of each
+// on the n x (2bw+1) band in shared memory, for half bands beyond kLuRowsMax (band_warp.cuh).  Step k computes the multiplier a_ik / a_kk of each
 // row below the pivot once (fac, at least bw entries), checks the column for a row swap, then
 // updates the trailing block one warp per row.  Every entry receives the same single update
 // per step as in the reference's row loop.  Returns 0 ok, 2 singular, 6 a row swap would be
@@ -133,7 +134,7 @@ __device__ int band_lu_smem(double* B, int n, int bw, int rw, double* fac) {
     for (int k = 0; k < n; ++k) {
         const int m = min(bw, n - 1 - k);
         const double akk = B[k * rw + bw];
-        const double aabs = fabs(akk);
+        const double aabs = fabs(akk), rkk = 1.0 / akk;
         int swap = 0, big = 0;
         for (int t = tid; t < m; t += nt) {
             const int i = k + 1 + t;
@@ -141,7 +142,7 @@ __device__ int band_lu_smem(double* B, int n, int bw, int rw, double* fac) {
             const double c = fabs(v);
             swap |= (c > aabs) ? 1 : 0;
             big |= (c > 1.0e-14) ? 1 : 0;
-            fac[t] = v / akk;
+            fac[t] = quot(v, akk, rkk);
         }
         // pivot search of linear_solver_backend.mojo:640-657: an entry strictly larger than
         // the diagonal selects another row; the largest candidate decides singularity
@@ -175,10 +176,10 @@ __device__ int band_chol_smem(double* B, int n, int bw, int rw, double* fac) {
         const int m = min(bw, n - 1 - k);
         const double dkk = B[k * rw + bw];
         if (!(dkk > 0.0)) return 2;
-        const double lkk = sqrt(dkk);
+        const double lkk = sqrt(dkk), rkk = 1.0 / lkk;
         for (int t = tid; t < m; t += nt) {
             const int i = k + 1 + t;
-            fac[t] = B[i * rw + (k - i + bw)] / lkk;
+            fac[t] = quot(B[i * rw + (k - i + bw)], lkk, rkk);
         }
         __syncthreads();
         for (int r = warp; r < m; r += nw) {
@@ -197,14 +198,17 @@ __device__ int band_chol_smem(double* B, int n, int bw, int rw, double* fac) {
 // BandGeneral forward/back substitution with one warp (_solve_band_general,
 // linear_solver_backend.mojo:735-770).  Forward: column-oriented, so row i receives
 // rhs_i - L_i,j0 w_j0 - L_i,j0+1 w_j0+1 - ... in increasing j, the order of the reference's row
-// loop.  Back: lane 0 runs each row's sum in the reference's order.  w may not alias rhs.
+// loop.  Back: band_back_warp for the bands it takes, else lane 0 runs each row's sum in the
+// reference's order.  w may not alias rhs; rhs null: w holds
+// the forward sweep's result already.  rd: n doubles of scratch.
 __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, int rw,
                                    const double* __restrict__ rhs, double* __restrict__ w,
-                                   double* __restrict__ x) {
+                                   double* __restrict__ x, double* __restrict__ rd) {
     const int lane = threadIdx.x & 31;
-    for (int i = lane; i < n; i += 32) w[i] = rhs[i];
+    if (rhs)
+        for (int i = lane; i < n; i += 32) w[i] = rhs[i];
     __syncwarp();
-    for (int j = 0; j < n; ++j) {
+    for (int j = 0; rhs && j < n; ++j) {
         const double wj = w[j];
         const int m = min(bw, n - 1 - j);
         for (int t = lane; t < m; t += 32) {
@@ -212,6 +216,10 @@ __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, 
             w[i] -= B[i * rw + (j - i + bw)] * wj;
         }
         __syncwarp();
+    }
+    if (bw <= kBackWarpMax) {
+        band_back_warp<false>(B, n, bw, rw, w, x, rd);
+        return;
     }
     if (lane == 0) {
         for (int i = n - 1; i >= 0; --i) {
@@ -228,7 +236,7 @@ __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, 
 // BandSPD substitution with one warp (_solve_band_spd, linear_solver_backend.mojo:772-812):
 // both sweeps are column-oriented, which is the reference's own order for each entry.
 __device__ void band_solve_chol_warp(const double* B, int n, int bw, int rw, const double* rhs,
-                                     double* w, double* x) {
+                                     double* w, double* x, double* rd) {
     const int lane = threadIdx.x & 31;
     for (int i = lane; i < n; i += 32) w[i] = rhs[i];
     __syncwarp();
@@ -243,6 +251,10 @@ __device__ void band_solve_chol_warp(const double* B, int n, int bw, int rw, con
             w[i] -= B[i * rw + (j - i + bw)] * wj;
         }
         __syncwarp();
+    }
+    if (bw <= kBackWarpMax) {
+        band_back_warp<true>(B, n, bw, rw, w, x, rd);
+        return;
     }
     for (int i = lane; i < n; i += 32) x[i] = w[i];
     __syncwarp();
@@ -531,6 +543,8 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
     __shared__ double red[32];
     __shared__ int red_r[32];
     __shared__ int s_it;  // this instance's Newton iterations of the step so far
+    __shared__ double s_rk[2], s_z[2];  // band_lu_cta
+    __shared__ int s_flag[2];
     const int inst = blockIdx.x;
     const int tid = threadIdx.x, nt = blockDim.x;
     {
@@ -747,6 +761,7 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
     bool dense = false;
     double* D = A.dense + I.dense_off;
     int* piv = A.piv + f0;
+    bool forward = false;  // w holds L^-1 R already
     if (!refresh) {
         // the step's factors
         dense = A.lu_dense[inst] != 0;
@@ -757,6 +772,13 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
         __syncthreads();
     } else if (I.spd) {
         rc = band_chol_smem(Kb, n, bw, rw, fac);
+    } else if (bw <= kLuRowsMax) {
+        for (int i = tid; i < n; i += nt) w[i] = R[i];
+        __syncthreads();
+        const int woff = (int)(w - Kb);
+        rc = modified ? band_lu_cta<true>(Kb, n, bw, rw, woff, s_rk, s_z, s_flag)
+                      : band_lu_cta<false>(Kb, n, bw, rw, woff, s_rk, s_z, s_flag);
+        forward = true;
     } else {
         rc = band_lu_smem(Kb, n, bw, rw, fac);
     }
@@ -810,9 +832,9 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
         if (dense)
             dense_solve_warp(D, piv, n, R, w, du);
         else if (I.spd)
-            band_solve_chol_warp(Kb, n, bw, rw, R, w, du);
+            band_solve_chol_warp(Kb, n, bw, rw, R, w, du, fac);
         else
-            band_solve_lu_warp(Kb, n, bw, rw, R, w, du);
+            band_solve_lu_warp(Kb, n, bw, rw, forward ? nullptr : R, w, du, fac);
     }
     __syncthreads();
     if (mode == INST_MODE_SOLVE_EXPORTED) {
