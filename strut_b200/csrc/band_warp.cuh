@@ -1,4 +1,4 @@
-// Band factor-solve in shared memory: the LU of narrow bands and the one-warp back substitution.
+// Band factor-solve in shared memory: the LU of narrow bands and the one-warp back substitutions.
 //
 // Algorithm (paths relative to the Strut project root):
 //   BandGeneral  src/mojo/solver/run_case/linear_solver_backend.mojo:631-680, 735-770
@@ -6,14 +6,17 @@
 //
 // A 2D frame's system (36 to 216 unknowns, half band 11 to 20) is a chain of n dependent steps of a
 // few hundred operations, so the time is the latency of a step.  Measured for 216 unknowns of half
-// band 20 (cycles per unknown): factorisation 1,230 -> 345, back substitution 810 -> 123.
+// band 20 (cycles per unknown): factorisation 1,230 -> 355, back substitution 810 -> 263 (the sums of a row
+// taken column by column instead, 123, rounded differently and were dropped: a batch of long records
+// is chaotic at the rounding level, and one record of 256 ended elsewhere).
 #pragma once
 
 #include <cstdint>
 
 namespace strut {
 
-constexpr int kBackWarpMax = 24;   // widest half band of band_back_warp: 24 + 8 rows in a warp's window
+constexpr int kBackWarpMax = 24;   // widest half band of the one-warp back substitutions: 24 + 8 rows in a
+                                   // warp's window
 constexpr int kBackWarpGroup = 8;  // unknowns per window position
 constexpr int kLuRowsMax = 62;     // widest half band of band_lu_cta
 constexpr int kLuRowsThreads = 256;
@@ -192,13 +195,65 @@ __device__ __forceinline__ int band_lu_cta(double* B, int n, int bw, int rw, int
     return band_lu_rows<8, 2, NW, KEEP>(B, n, bw, rw, woff, rk, z, flag);
 }
 
-// Back substitution with one warp for bw <= kBackWarpMax: x from U x = w (LU) or L^T x = w (CHOL),
-// column by column from the end (a lane per row of the window, so that only a product and a
-// shuffle separate one unknown from the next; the row sums of the reference run through all bw
-// terms in between).  The quotient by the diagonal is formed from its reciprocal, computed ahead,
-// and one correction step.  rd: n doubles of scratch.
-template <bool CHOL>
-__device__ __noinline__ void band_back_warp(const double* B, int n, int bw, int rw, const double* w, double* x,
+// U x = w with one warp for bw <= kBackWarpMax, every row's sum in the reference's order (columns
+// upwards from the diagonal, so the chain of a row runs through all its bw products, the newest
+// unknown's first).  The unknowns a row needs and the next row's entries are in registers, so a row
+// costs its chain and a quotient (bw 20: 263 cycles; one lane with its operands in shared memory
+// took 810).  EXACT: bw == BW; else bw <= BW.  Slots of columns outside the matrix hold zeros.
+// rd: n doubles of scratch.
+template <int BW, bool EXACT>
+__device__ __noinline__ void band_back_lu(const double* B, int n, int bw, int rw, const double* w, double* x,
+                                          double* rd) {
+    const int lane = threadIdx.x & 31;
+    for (int i = lane; i < n; i += 32) rd[i] = 1.0 / B[i * rw + bw];
+    __syncwarp();
+    double xw[BW], u[BW];  // x_(i + 1 + t), U(i, i + 1 + t)
+    const double* row = B + (n - 1) * rw + bw;
+#pragma unroll
+    for (int t = 0; t < BW; ++t) {
+        xw[t] = 0.0;
+        u[t] = EXACT || t < bw ? row[1 + t] : 0.0;
+    }
+    double s = w[n - 1], d = row[0], r = rd[n - 1];
+#pragma unroll 2
+    for (int i = n - 1; i >= 0; --i) {
+        const int ip = i > 0 ? i - 1 : 0;
+        row = B + ip * rw + bw;
+        double un[BW];
+#pragma unroll
+        for (int t = 0; t < BW; ++t) un[t] = EXACT || t < bw ? row[1 + t] : 0.0;
+        const double sn = w[ip], dn = row[0], rn = rd[ip];
+#pragma unroll
+        for (int t = 0; t < BW; ++t) s -= u[t] * xw[t];
+        s = quot(s, d, r);
+        if (lane == 0) x[i] = s;
+#pragma unroll
+        for (int t = BW - 1; t > 0; --t) xw[t] = xw[t - 1];
+        xw[0] = s;
+#pragma unroll
+        for (int t = 0; t < BW; ++t) u[t] = un[t];
+        s = sn;
+        d = dn;
+        r = rn;
+    }
+    __syncwarp();
+}
+
+// The half bands of 2D frames of two to five bays have their own instance.
+__device__ __forceinline__ void band_back_lu_any(const double* B, int n, int bw, int rw, const double* w, double* x,
+                                                 double* rd) {
+    if (bw == 11) band_back_lu<11, true>(B, n, bw, rw, w, x, rd);
+    else if (bw == 14) band_back_lu<14, true>(B, n, bw, rw, w, x, rd);
+    else if (bw == 17) band_back_lu<17, true>(B, n, bw, rw, w, x, rd);
+    else if (bw == 20) band_back_lu<20, true>(B, n, bw, rw, w, x, rd);
+    else if (bw <= 12) band_back_lu<12, false>(B, n, bw, rw, w, x, rd);
+    else band_back_lu<kBackWarpMax, false>(B, n, bw, rw, w, x, rd);
+}
+
+// L^T x = w with one warp for bw <= kBackWarpMax, column by column from the end (the reference's
+// order), a lane per row of the window, so that only a quotient and a shuffle separate one unknown
+// from the next.  rd: n doubles of scratch.
+__device__ __noinline__ void band_back_chol(const double* B, int n, int bw, int rw, const double* w, double* x,
                                             double* rd) {
     constexpr unsigned all = 0xffffffffu;
     constexpr int G = kBackWarpGroup;
@@ -208,8 +263,7 @@ __device__ __noinline__ void band_back_warp(const double* B, int n, int bw, int 
     int j0 = n - 1;
     int row = j0 - ((j0 - lane) & 31);
     auto coef = [&](int r, int j) -> double {
-        if (r < 0 || r >= j || r < j - bw) return 0.0;
-        return CHOL ? B[j * rw + (r - j + bw)] : B[r * rw + (j - r + bw)];
+        return r < 0 || r >= j || r < j - bw ? 0.0 : B[j * rw + (r - j + bw)];
     };
     double c[G], v, r = 0.0, d = 1.0;
 #pragma unroll

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
     double* w = R + n;
     double* xs = w + n;
     double* fac = xs + n;
-    // (the slots of columns outside the matrix are never used)
+    // (columns before the first are never used, those behind the last have to be zeros)
     if (!spd) {
 #pragma unroll 8
         for (int t = tid; t < n * rw; t += nt) Kb[t] = band[t];
@@ -55,6 +55,10 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
         }
     }
     for (int i = tid; i < n; i += nt) R[i] = rhs[i];
+    __syncthreads();
+    if (!spd)
+        for (int i = n - bw + tid; i < n; i += nt)
+            for (int j = n; j <= i + bw; ++j) Kb[i * rw + bw + j - i] = 0.0;
     __syncthreads();
     bool forward = false;  // w holds L^-1 rhs already
     int rc;

@@ -198,8 +198,8 @@ __device__ int band_chol_smem(double* B, int n, int bw, int rw, double* fac) {
 // BandGeneral forward/back substitution with one warp (_solve_band_general,
 // linear_solver_backend.mojo:735-770).  Forward: column-oriented, so row i receives
 // rhs_i - L_i,j0 w_j0 - L_i,j0+1 w_j0+1 - ... in increasing j, the order of the reference's row
-// loop.  Back: band_back_warp for the bands it takes, else lane 0 runs each row's sum in the
-// reference's order.  w may not alias rhs; rhs null: w holds
+// loop.  Back: each row's sum in the reference's order, by band_back_lu for the bands it takes,
+// else by lane 0.  w may not alias rhs; rhs null: w holds
 // the forward sweep's result already.  rd: n doubles of scratch.
 __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, int rw,
                                    const double* __restrict__ rhs, double* __restrict__ w,
@@ -218,7 +218,7 @@ __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, 
         __syncwarp();
     }
     if (bw <= kBackWarpMax) {
-        band_back_warp<false>(B, n, bw, rw, w, x, rd);
+        band_back_lu_any(B, n, bw, rw, w, x, rd);
         return;
     }
     if (lane == 0) {
@@ -253,7 +253,7 @@ __device__ void band_solve_chol_warp(const double* B, int n, int bw, int rw, con
         __syncwarp();
     }
     if (bw <= kBackWarpMax) {
-        band_back_warp<true>(B, n, bw, rw, w, x, rd);
+        band_back_chol(B, n, bw, rw, w, x, rd);
         return;
     }
     for (int i = lane; i < n; i += 32) x[i] = w[i];
