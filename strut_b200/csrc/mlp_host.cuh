@@ -93,11 +93,10 @@ struct StrutMlp {
     float *d_b1 = nullptr, *d_b2 = nullptr, *d_b3 = nullptr;
     int* d_err = nullptr;
     long long adam_step = 0;
+    Arena mem;  // on the legacy default stream
     ~StrutMlp() {
-        for (void* p : {(void*)d_params, (void*)d_m, (void*)d_v, (void*)d_w1t, (void*)d_w2t, (void*)d_w3t,
-                        (void*)d_w2, (void*)d_w3,
-                        (void*)d_b1, (void*)d_b2, (void*)d_b3, (void*)d_err})
-            if (p) cudaFree(p);
+        cudaDeviceSynchronize();  // an analysis may have run the network on its own stream
+        mem.release();
     }
     int n_params() const { return n_in * kMlpH + kMlpH + kMlpH * kMlpH + kMlpH + kMlpH * n_out + n_out; }
     strut::MlpDev dev() const { return strut::MlpDev{d_w1t, d_w2t, d_w3t, d_b1, d_b2, d_b3}; }
@@ -119,7 +118,7 @@ int mlp_pack(StrutMlp* m, cudaStream_t s) {
 int mlp_forward_dev(StrutMlp* m, const float* d_x, int n, float* d_y, cudaStream_t s) {
     const int n_tiles = (n + strut::kMlpTile - 1) / strut::kMlpTile;
     __nv_bfloat16* d_xt = nullptr;
-    CK(cudaMallocAsync((void**)&d_xt, (size_t)n_tiles * strut::kMlpBytesX, s));
+    TRY(pool_alloc((void**)&d_xt, (size_t)n_tiles * strut::kMlpBytesX, s));
     const long long tot = (long long)n_tiles * strut::kMlpTile * strut::kMlpKin;
     strut::mlp_pack_x_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(d_x, n, m->n_in, d_xt, n_tiles);
     CK(cudaGetLastError());
@@ -169,22 +168,15 @@ int strut_gpu_mlp_create(int32_t n_in, int32_t n_out, StrutMlp** out) {
     };
     if (cudaGetDevice(&m->device) != cudaSuccess) return bail(fail(STRUT_CUDA_ERROR, "no device"));
     const size_t np = (size_t)m->n_params();
-    if (cudaMalloc((void**)&m->d_params, np * 4) != cudaSuccess || cudaMalloc((void**)&m->d_m, np * 4) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_v, np * 4) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_w1t, strut::kMlpBytesW1) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_w2t, strut::kMlpBytesW2) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_w3t, strut::kMlpBytesW3) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_w2, strut::kMlpBytesW2) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_w3, strut::kMlpBytesW3) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_b1, strut::kMlpH * 4) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_b2, strut::kMlpH * 4) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_b3, strut::kMlpNout * 4) != cudaSuccess ||
-        cudaMalloc((void**)&m->d_err, sizeof(int)) != cudaSuccess)
-        return bail(fail(STRUT_CUDA_ERROR, "device allocation failed"));
-    cudaMemset(m->d_params, 0, np * 4);
-    cudaMemset(m->d_m, 0, np * 4);
-    cudaMemset(m->d_v, 0, np * 4);
-    cudaMemset(m->d_err, 0, sizeof(int));
+    Arena& al = m->mem;
+    int rc = STRUT_OK;
+    if ((rc = dzeros(&m->d_params, np, al)) || (rc = dzeros(&m->d_m, np, al)) || (rc = dzeros(&m->d_v, np, al)) ||
+        (rc = dzeros(&m->d_w1t, strut::kMlpBytesW1 / 2, al)) || (rc = dzeros(&m->d_w2t, strut::kMlpBytesW2 / 2, al)) ||
+        (rc = dzeros(&m->d_w3t, strut::kMlpBytesW3 / 2, al)) || (rc = dzeros(&m->d_w2, strut::kMlpBytesW2 / 2, al)) ||
+        (rc = dzeros(&m->d_w3, strut::kMlpBytesW3 / 2, al)) || (rc = dzeros(&m->d_b1, strut::kMlpH, al)) ||
+        (rc = dzeros(&m->d_b2, strut::kMlpH, al)) || (rc = dzeros(&m->d_b3, strut::kMlpNout, al)) ||
+        (rc = dzeros(&m->d_err, 1, al)))
+        return bail(rc);
     if (cudaFuncSetAttribute(strut::mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)strut::kMlpFwdSmem) != cudaSuccess ||
         cudaFuncSetAttribute(strut::mlp_train_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -229,14 +221,14 @@ int strut_gpu_mlp_loss_grad(StrutMlp* m, const float* x, const float* t, int32_t
     for (int i = 0; i < n; ++i) idx[i] = i;
     int rc = STRUT_OK;
     auto run = [&]() -> int {
-        CK(cudaMalloc((void**)&d_x, (size_t)n * m->n_in * 4));
-        CK(cudaMalloc((void**)&d_t, (size_t)n * m->n_out * 4));
-        CK(cudaMalloc((void**)&d_tb, (size_t)n * m->n_out * 4));
-        CK(cudaMalloc((void**)&d_idx, (size_t)n * 4));
-        CK(cudaMalloc((void**)&d_xt, (size_t)n_tiles * strut::kMlpBytesX));
-        CK(cudaMalloc((void**)&d_part, (size_t)n_tiles * np * 4));
-        CK(cudaMalloc((void**)&d_sse, (size_t)n_tiles * 8));
-        CK(cudaMalloc((void**)&d_g, (size_t)np * 4));
+        TRY(pool_alloc((void**)&d_x, (size_t)n * m->n_in * 4, nullptr));
+        TRY(pool_alloc((void**)&d_t, (size_t)n * m->n_out * 4, nullptr));
+        TRY(pool_alloc((void**)&d_tb, (size_t)n * m->n_out * 4, nullptr));
+        TRY(pool_alloc((void**)&d_idx, (size_t)n * 4, nullptr));
+        TRY(pool_alloc((void**)&d_xt, (size_t)n_tiles * strut::kMlpBytesX, nullptr));
+        TRY(pool_alloc((void**)&d_part, (size_t)n_tiles * np * 4, nullptr));
+        TRY(pool_alloc((void**)&d_sse, (size_t)n_tiles * 8, nullptr));
+        TRY(pool_alloc((void**)&d_g, (size_t)np * 4, nullptr));
         CK(cudaMemcpy(d_x, x, (size_t)n * m->n_in * 4, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_t, t, (size_t)n * m->n_out * 4, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_idx, idx.data(), (size_t)n * 4, cudaMemcpyHostToDevice));
@@ -261,7 +253,7 @@ int strut_gpu_mlp_loss_grad(StrutMlp* m, const float* x, const float* t, int32_t
     rc = run();
     for (void* p : {(void*)d_x, (void*)d_t, (void*)d_tb, (void*)d_idx, (void*)d_xt, (void*)d_part, (void*)d_sse,
                     (void*)d_g})
-        if (p) cudaFree(p);
+        if (p) cudaFreeAsync(p, nullptr);
     return rc;
 }
 
@@ -275,13 +267,13 @@ int strut_gpu_mlp_train(StrutMlp* m, const float* x, const float* t, int32_t n, 
     double* d_sse = nullptr;
     __nv_bfloat16* d_xt = nullptr;
     auto run = [&]() -> int {
-        CK(cudaMalloc((void**)&d_x, (size_t)n * m->n_in * 4));
-        CK(cudaMalloc((void**)&d_t, (size_t)n * m->n_out * 4));
-        CK(cudaMalloc((void**)&d_tb, (size_t)batch * m->n_out * 4));
-        CK(cudaMalloc((void**)&d_idx, (size_t)n * 4));
-        CK(cudaMalloc((void**)&d_xt, (size_t)max_tiles * strut::kMlpBytesX));
-        CK(cudaMalloc((void**)&d_part, (size_t)max_tiles * np * 4));
-        CK(cudaMalloc((void**)&d_sse, (size_t)max_tiles * 8));
+        TRY(pool_alloc((void**)&d_x, (size_t)n * m->n_in * 4, nullptr));
+        TRY(pool_alloc((void**)&d_t, (size_t)n * m->n_out * 4, nullptr));
+        TRY(pool_alloc((void**)&d_tb, (size_t)batch * m->n_out * 4, nullptr));
+        TRY(pool_alloc((void**)&d_idx, (size_t)n * 4, nullptr));
+        TRY(pool_alloc((void**)&d_xt, (size_t)max_tiles * strut::kMlpBytesX, nullptr));
+        TRY(pool_alloc((void**)&d_part, (size_t)max_tiles * np * 4, nullptr));
+        TRY(pool_alloc((void**)&d_sse, (size_t)max_tiles * 8, nullptr));
         CK(cudaMemcpy(d_x, x, (size_t)n * m->n_in * 4, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_t, t, (size_t)n * m->n_out * 4, cudaMemcpyHostToDevice));
         CK(cudaMemset(m->d_err, 0, sizeof(int)));
@@ -319,15 +311,15 @@ int strut_gpu_mlp_train(StrutMlp* m, const float* x, const float* t, int32_t n, 
     };
     const int rc = run();
     for (void* p : {(void*)d_x, (void*)d_t, (void*)d_tb, (void*)d_idx, (void*)d_xt, (void*)d_part, (void*)d_sse})
-        if (p) cudaFree(p);
+        if (p) cudaFreeAsync(p, nullptr);
     return rc;
 }
 
 int strut_gpu_mlp_forward(StrutMlp* m, const float* x, int32_t n, float* y) {
     if (!m || !x || !y || n < 1) return fail(STRUT_BAD_ARG, "bad arguments");
     float *d_x = nullptr, *d_y = nullptr;
-    CK(cudaMalloc((void**)&d_x, (size_t)n * m->n_in * 4));
-    CK(cudaMalloc((void**)&d_y, (size_t)n * m->n_out * 4));
+    TRY(pool_alloc((void**)&d_x, (size_t)n * m->n_in * 4, nullptr));
+    TRY(pool_alloc((void**)&d_y, (size_t)n * m->n_out * 4, nullptr));
     CK(cudaMemcpy(d_x, x, (size_t)n * m->n_in * 4, cudaMemcpyHostToDevice));
     CK(cudaMemset(m->d_err, 0, sizeof(int)));
     int rc = mlp_forward_dev(m, d_x, n, d_y, 0);
@@ -338,8 +330,8 @@ int strut_gpu_mlp_forward(StrutMlp* m, const float* x, int32_t n, float* y) {
         if (err) rc = fail(STRUT_CUDA_ERROR, "network kernel wait ran out");
         else CK(cudaMemcpy(y, d_y, (size_t)n * m->n_out * 4, cudaMemcpyDeviceToHost));
     }
-    cudaFree(d_x);
-    cudaFree(d_y);
+    cudaFreeAsync(d_x, nullptr);
+    cudaFreeAsync(d_y, nullptr);
     return rc;
 }
 

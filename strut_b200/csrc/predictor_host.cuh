@@ -6,7 +6,7 @@ struct PredState {
     StrutMlp* mlp = nullptr;  // not owned
     strut::PredDev P{};
     int n_tiles = 0;
-    std::vector<void*> allocs;
+    Arena mem;  // on the handle's stream
     float* d_x = nullptr;
     __nv_bfloat16* d_xt = nullptr;
     float* d_y = nullptr;
@@ -14,9 +14,7 @@ struct PredState {
     int* d_rejected = nullptr;
     int* d_skip = nullptr;
     bool owns_base = false;  // u_base / estate_base were allocated for the predictor
-    ~PredState() {
-        for (void* p : allocs) cudaFree(p);
-    }
+    ~PredState() { mem.release(); }
 };
 
 static void pred_free(PredState* p) { delete p; }
@@ -25,10 +23,7 @@ namespace {
 
 template <typename T>
 int pred_alloc(PredState* ps, T** p, size_t n) {
-    CK(cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T)));
-    CK(cudaMemset(*p, 0, std::max<size_t>(n, 1) * sizeof(T)));
-    ps->allocs.push_back(*p);
-    return STRUT_OK;
+    return dzeros(p, n, ps->mem);
 }
 
 
@@ -113,6 +108,7 @@ int strut_gpu_set_predictor(StrutHandle* h, StrutMlp* m, const float* x_mean, co
                                        std::to_string(ndf) + " outputs");
     if (!x_mean || !x_scale || !y_scale) return fail(STRUT_BAD_ARG, "normalisation arrays required");
     PredState* ps = new PredState();
+    ps->mem.s = h->stream;
     ps->mlp = m;
     const int nn = (int)h->pn_inst.size();
     ps->n_tiles = (nn + kMlpTile - 1) / kMlpTile;
@@ -162,7 +158,7 @@ int strut_gpu_set_predictor(StrutHandle* h, StrutMlp* m, const float* x_mean, co
         ps->owns_base = true;
     }
     auto up = [&](void* dst, const void* src, size_t bytes) -> int {
-        CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream));
         return STRUT_OK;
     };
     if ((rc = up(d_nf, h->pn_free.data(), h->pn_free.size() * 4)) || (rc = up(d_ni, h->pn_inst.data(), (size_t)nn * 4)) ||

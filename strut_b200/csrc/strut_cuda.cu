@@ -27,6 +27,7 @@
 #include "element_kernels.cuh"
 #include "kat_kernels.cuh"
 #include "fiber_stream_kernels.cuh"
+#include "init_kernels.cuh"
 #include "solver_kernels.cuh"
 #include "largeband_kernels.cuh"
 #include "shell_kernels.cuh"
@@ -243,24 +244,6 @@ double path_eval(const StrutExcitation& x, double t) {
     return x.factor * (v1 + (v2 - v1) * (incr - (double)incr1));
 }
 
-template <typename T>
-int upload(T** dptr, const std::vector<T>& h, std::vector<void*>& allocs) {
-    const size_t n = std::max<size_t>(h.size(), 1);
-    CK(cudaMalloc((void**)dptr, n * sizeof(T)));
-    allocs.push_back(*dptr);
-    if (!h.empty()) CK(cudaMemcpy(*dptr, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return STRUT_OK;
-}
-
-template <typename T>
-int dzeros(T** dptr, size_t n, std::vector<void*>& allocs) {
-    n = std::max<size_t>(n, 1);
-    CK(cudaMalloc((void**)dptr, n * sizeof(T)));
-    allocs.push_back(*dptr);
-    CK(cudaMemset(*dptr, 0, n * sizeof(T)));
-    return STRUT_OK;
-}
-
 #define TRY(x)                       \
     do {                             \
         int rc_ = (x);               \
@@ -268,6 +251,8 @@ int dzeros(T** dptr, size_t n, std::vector<void*>& allocs) {
     } while (0)
 
 }  // namespace
+
+#include "device_memory.cuh"
 
 struct ExcHost {
     int num;
@@ -279,7 +264,7 @@ struct StrutHandle {
     int n_inst = 0;
     int device = 0;
     cudaStream_t stream = nullptr;
-    std::vector<void*> allocs;
+    Arena mem;  // every array that lives as long as the handle (on stream)
     std::vector<DevInst> insts;
     std::vector<ExcHost> exc;
     std::vector<int> rec_off, n_rec, rece_off, n_rece;
@@ -345,7 +330,6 @@ struct StrutHandle {
     int* d_hist_iters = nullptr;
     int hist_cap = 0;
     int steps_done = 0;
-    int* h_ctrl = nullptr;  // pinned: nactive
     bool state_determined = false;
     bool prof = false;
     StrutKernelProfile P;
@@ -371,13 +355,10 @@ struct StrutHandle {
     int graph_tune_gen = -1;
     ~StrutHandle();
     void release() {
-        for (void* p : allocs) cudaFree(p);
-        if (d_hist_disp) cudaFree(d_hist_disp);
-        if (d_hist_ef) cudaFree(d_hist_ef);
-        if (d_hist_iters) cudaFree(d_hist_iters);
-        if (d_hist_sec) cudaFree(d_hist_sec);
-        if (d_ag) cudaFree(d_ag);
-        if (h_ctrl) cudaFreeHost(h_ctrl);
+        if (stream) cudaStreamSynchronize(stream);
+        mem.release();
+        for (void* p : {(void*)d_hist_disp, (void*)d_hist_ef, (void*)d_hist_iters, (void*)d_hist_sec, (void*)d_ag})
+            if (p) cudaFreeAsync(p, stream);
         if (gexec) cudaGraphExecDestroy(gexec);
         if (graph) cudaGraphDestroy(graph);
         if (ev0) cudaEventDestroy(ev0);
@@ -565,26 +546,30 @@ static int ensure_history(StrutHandle* h, int need) {
     int* ni = nullptr;
     double* ns = nullptr;
     const int sw = h->ndf_all == 6 ? 4 : 2;
-    CK(cudaMalloc((void**)&ns, (size_t)cap * std::max(h->n_sec_slots, 1) * sw * sizeof(double)));
-    CK(cudaMalloc((void**)&nd, (size_t)cap * std::max(h->n_rec_total, 1) * sizeof(double)));
-    CK(cudaMalloc((void**)&ne, (size_t)cap * std::max(h->n_rece_slots, 1) * h->ef_w * sizeof(double)));
-    CK(cudaMalloc((void**)&ni, (size_t)cap * h->n_inst * sizeof(int)));
-    CK(cudaMemset(ni, 0, (size_t)cap * h->n_inst * sizeof(int)));
+    const size_t bs = (size_t)std::max(h->n_sec_slots, 1) * sw * sizeof(double);
+    const size_t bd = (size_t)std::max(h->n_rec_total, 1) * sizeof(double);
+    const size_t be = (size_t)std::max(h->n_rece_slots, 1) * h->ef_w * sizeof(double);
+    const size_t bi = (size_t)h->n_inst * sizeof(int);
+    const cudaStream_t s = h->stream;
+    TRY(pool_alloc((void**)&ns, cap * bs, s));
+    TRY(pool_alloc((void**)&nd, cap * bd, s));
+    TRY(pool_alloc((void**)&ne, cap * be, s));
+    TRY(pool_alloc((void**)&ni, cap * bi, s));
+    // (an instance that has failed records nothing more: its rows stay zero)
+    CK(cudaMemsetAsync(ns, 0, cap * bs, s));
+    CK(cudaMemsetAsync(nd, 0, cap * bd, s));
+    CK(cudaMemsetAsync(ne, 0, cap * be, s));
+    CK(cudaMemsetAsync(ni, 0, cap * bi, s));
     if (h->hist_cap > 0 && h->steps_done > 0) {
-        CK(cudaMemcpy(nd, h->d_hist_disp, (size_t)h->steps_done * std::max(h->n_rec_total, 1) * sizeof(double),
-                      cudaMemcpyDeviceToDevice));
-        CK(cudaMemcpy(ne, h->d_hist_ef, (size_t)h->steps_done * std::max(h->n_rece_slots, 1) * h->ef_w * sizeof(double),
-                      cudaMemcpyDeviceToDevice));
-        CK(cudaMemcpy(ni, h->d_hist_iters, (size_t)h->steps_done * h->n_inst * sizeof(int),
-                      cudaMemcpyDeviceToDevice));
-        CK(cudaMemcpy(ns, h->d_hist_sec, (size_t)h->steps_done * std::max(h->n_sec_slots, 1) * sw * sizeof(double),
-                      cudaMemcpyDeviceToDevice));
+        const size_t S = h->steps_done;
+        CK(cudaMemcpyAsync(nd, h->d_hist_disp, S * bd, cudaMemcpyDeviceToDevice, s));
+        CK(cudaMemcpyAsync(ne, h->d_hist_ef, S * be, cudaMemcpyDeviceToDevice, s));
+        CK(cudaMemcpyAsync(ni, h->d_hist_iters, S * bi, cudaMemcpyDeviceToDevice, s));
+        CK(cudaMemcpyAsync(ns, h->d_hist_sec, S * bs, cudaMemcpyDeviceToDevice, s));
     }
-    if (h->d_hist_sec) cudaFree(h->d_hist_sec);
+    for (void* p : {(void*)h->d_hist_sec, (void*)h->d_hist_disp, (void*)h->d_hist_ef, (void*)h->d_hist_iters})
+        if (p) CK(cudaFreeAsync(p, s));
     h->d_hist_sec = ns;
-    if (h->d_hist_disp) cudaFree(h->d_hist_disp);
-    if (h->d_hist_ef) cudaFree(h->d_hist_ef);
-    if (h->d_hist_iters) cudaFree(h->d_hist_iters);
     h->d_hist_disp = nd;
     h->d_hist_ef = ne;
     h->d_hist_iters = ni;
@@ -770,7 +755,10 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         delete h;
         return code;
     };
-    CK(cudaGetDevice(&h->device));
+    if (cudaGetDevice(&h->device) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
+        return bail(fail(STRUT_CUDA_ERROR, "cannot create the handle's stream"));
+    h->mem.s = h->stream;
     h->n_inst = num_instances;
     std::vector<DevMat> mats;
     SectionPack sp;
@@ -1092,107 +1080,81 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             }
         }
         const int rw = 2 * bw + 1;
+        std::vector<std::pair<int, double>> rows;
         // band slot contributions, element order (stiffness_internal_frame2d.mojo:594-619)
-        std::vector<std::vector<int>> slots((size_t)nf * rw);
-        std::vector<std::vector<int>> fcontr(nf);
-        std::vector<std::vector<double>> slotc, fc;
-        if (any_mpc) {
-            slotc.resize((size_t)nf * rw);
-            fc.resize(nf);
+        // retained free dofs and coefficients of every dof (rows_of), as one list
+        std::vector<int> term_ptr(d.num_dofs + 1, 0), term_dof;
+        std::vector<double> term_coef;
+        for (int dof = 0; dof < d.num_dofs; ++dof) {
+            rows_of(dof, rows);
+            for (auto& t : rows)
+                if (t.first >= 0 && t.second != 0.0) {
+                    term_dof.push_back(t.first);
+                    term_coef.push_back(t.second);
+                }
+            term_ptr[dof + 1] = (int)term_dof.size();
         }
-        if (d.num_slaves == 0) {
-            for (int e = 0; e < d.num_elements; ++e) {
-                const DevElem& E = elems[e0 + e];
-                for (int a = 0; a < nd; ++a) {
-                    const int ia = efree[(size_t)nd * e + a];
-                    if (ia < 0) continue;
-                    for (int b = 0; b < nd; ++b) {
-                        const int ib = efree[(size_t)nd * e + b];
-                        if (ib < 0) continue;
-                        const size_t sl = (size_t)ia * rw + (ib - ia + bw);
-                        slots[sl].push_back((int)(E.ek_off + a * nd + b));
-                        if (any_mpc) slotc[sl].push_back(1.0);
-                    }
-                    fcontr[ia].push_back((int)(E.ef_off + a));
-                    if (any_mpc) fc[ia].push_back(1.0);
+        // every contribution in assembly order: on_k(slot, index into ek, coefficient) and
+        // on_f(free dof, index into ef, coefficient).  Constrained dofs are collapsed (c_i k c_j onto
+        // the retained free dofs); entries outside the half width detected from the elements' free
+        // dofs are dropped, as Strut's band load drops them (linear_solver_backend.mojo:413-427)
+        auto element_terms = [&](const int32_t* dofs, int ndl, long long ek0, long long ef0, auto&& on_k, auto&& on_f) {
+            for (int a = 0; a < ndl; ++a) {
+                const int a0 = term_ptr[dofs[a]], a1 = term_ptr[dofs[a] + 1];
+                for (int b = 0; a0 < a1 && b < ndl; ++b) {
+                    const int b0 = term_ptr[dofs[b]], b1 = term_ptr[dofs[b] + 1];
+                    for (int ta = a0; ta < a1; ++ta)
+                        for (int tb = b0; tb < b1; ++tb) {
+                            const int o = term_dof[tb] - term_dof[ta];
+                            if (std::abs(o) > bw) continue;
+                            on_k((size_t)term_dof[ta] * rw + (o + bw), (int)(ek0 + a * ndl + b),
+                                 term_coef[ta] * term_coef[tb]);
+                        }
                 }
+                for (int ta = a0; ta < a1; ++ta) on_f(term_dof[ta], (int)(ef0 + a), term_coef[ta]);
             }
-            for (int s = 0; s < d.num_shells; ++s) {
-                const DevShell& S = h->shells_h[sh0 + s];
-                for (int a = 0; a < 24; ++a) {
-                    const int ia = sfree[(size_t)24 * s + a];
-                    if (ia < 0) continue;
-                    for (int b = 0; b < 24; ++b) {
-                        const int ib = sfree[(size_t)24 * s + b];
-                        if (ib < 0) continue;
-                        const size_t sl = (size_t)ia * rw + (ib - ia + bw);
-                        slots[sl].push_back((int)(S.ek_off + a * 24 + b));
-                        if (any_mpc) slotc[sl].push_back(1.0);
-                    }
-                    fcontr[ia].push_back((int)(S.ef_off + a));
-                    if (any_mpc) fc[ia].push_back(1.0);
-                }
-            }
-        } else {
-            // collapse c_i k c_j onto the retained free dofs; entries outside the half width
-            // detected from the elements' free dofs are dropped, as Strut's band load drops
-            // them (linear_solver_backend.mojo:413-427)
-            std::vector<std::pair<int, double>> ra, rb;
-            for (int e = 0; e < d.num_elements; ++e) {
-                const DevElem& E = elems[e0 + e];
-                for (int a = 0; a < nd; ++a) {
-                    rows_of(d.elements[e].dof[a], ra);
-                    for (int b = 0; b < nd; ++b) {
-                        rows_of(d.elements[e].dof[b], rb);
-                        for (auto& ta : ra)
-                            for (auto& tb : rb) {
-                                if (ta.first < 0 || tb.first < 0 || std::abs(ta.first - tb.first) > bw) continue;
-                                if (ta.second == 0.0 || tb.second == 0.0) continue;
-                                const size_t sl = (size_t)ta.first * rw + (tb.first - ta.first + bw);
-                                slots[sl].push_back((int)(E.ek_off + a * nd + b));
-                                slotc[sl].push_back(ta.second * tb.second);
-                            }
-                    }
-                    for (auto& ta : ra) {
-                        if (ta.first < 0 || ta.second == 0.0) continue;
-                        fcontr[ta.first].push_back((int)(E.ef_off + a));
-                        fc[ta.first].push_back(ta.second);
-                    }
-                }
-            }
-            for (int s = 0; s < d.num_shells; ++s) {
-                const DevShell& S = h->shells_h[sh0 + s];
-                for (int a = 0; a < 24; ++a) {
-                    rows_of(d.shells[s].dof[a], ra);
-                    for (int b = 0; b < 24; ++b) {
-                        rows_of(d.shells[s].dof[b], rb);
-                        for (auto& ta : ra)
-                            for (auto& tb : rb) {
-                                if (ta.first < 0 || tb.first < 0 || std::abs(ta.first - tb.first) > bw) continue;
-                                if (ta.second == 0.0 || tb.second == 0.0) continue;
-                                const size_t sl = (size_t)ta.first * rw + (tb.first - ta.first + bw);
-                                slots[sl].push_back((int)(S.ek_off + a * 24 + b));
-                                slotc[sl].push_back(ta.second * tb.second);
-                            }
-                    }
-                    for (auto& ta : ra) {
-                        if (ta.first < 0 || ta.second == 0.0) continue;
-                        fcontr[ta.first].push_back((int)(S.ef_off + a));
-                        fc[ta.first].push_back(ta.second);
-                    }
-                }
-            }
+        };
+        auto all_terms = [&](auto&& on_k, auto&& on_f) {
+            for (int e = 0; e < d.num_elements; ++e)
+                element_terms(d.elements[e].dof, nd, elems[e0 + e].ek_off, elems[e0 + e].ef_off, on_k, on_f);
+            for (int s = 0; s < d.num_shells; ++s)
+                element_terms(d.shells[s].dof, 24, h->shells_h[sh0 + s].ek_off, h->shells_h[sh0 + s].ef_off, on_k,
+                              on_f);
+        };
+        // count, then place: each slot's and each dof's contributions end up in assembly order
+        const size_t k0 = slot_contrib.size(), f0 = fint_contrib.size();
+        std::vector<int> nk((size_t)nf * rw, 0), nfc(nf, 0);
+        all_terms([&](size_t sl, int, double) { ++nk[sl]; }, [&](int r, int, double) { ++nfc[r]; });
+        std::vector<size_t> at_k((size_t)nf * rw), at_f(nf);
+        size_t pos = k0;
+        for (size_t k = 0; k < nk.size(); ++k) {
+            at_k[k] = pos;
+            pos += nk[k];
+            slot_ptr.push_back((long long)pos);
         }
-        for (size_t k = 0; k < slots.size(); ++k) {
-            slot_contrib.insert(slot_contrib.end(), slots[k].begin(), slots[k].end());
-            if (any_mpc) slot_coef.insert(slot_coef.end(), slotc[k].begin(), slotc[k].end());
-            slot_ptr.push_back((long long)slot_contrib.size());
-        }
+        slot_contrib.resize(pos);
+        if (any_mpc) slot_coef.resize(pos);
+        const size_t ncontrib = pos - k0;
+        pos = f0;
         for (int k = 0; k < nf; ++k) {
-            fint_contrib.insert(fint_contrib.end(), fcontr[k].begin(), fcontr[k].end());
-            if (any_mpc) fint_coef.insert(fint_coef.end(), fc[k].begin(), fc[k].end());
-            fint_ptr.push_back((int)fint_contrib.size());
+            at_f[k] = pos;
+            pos += nfc[k];
+            fint_ptr.push_back((int)pos);
         }
+        fint_contrib.resize(pos);
+        if (any_mpc) fint_coef.resize(pos);
+        const size_t nfcontrib = pos - f0;
+        all_terms(
+            [&](size_t sl, int idx, double c) {
+                const size_t at = at_k[sl]++;
+                slot_contrib[at] = idx;
+                if (any_mpc) slot_coef[at] = c;
+            },
+            [&](int r, int idx, double c) {
+                const size_t at = at_f[r]++;
+                fint_contrib[at] = idx;
+                if (any_mpc) fint_coef[at] = c;
+            });
         DevInst I;
         std::memset(&I, 0, sizeof(I));
         I.sl_off = sl0;
@@ -1272,10 +1234,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         {
             // gathered element k / f entries, the band written to shared memory is not HBM;
             // K_init band, the gather lists, and the free-dof vectors
-            long long ncontrib = 0, nfc = 0;
-            for (auto& v : slots) ncontrib += (long long)v.size();
-            for (auto& v : fcontr) nfc += (long long)v.size();
-            I.io_bytes = 12.0 * ncontrib + 12.0 * nfc + 8.0 * (double)nf * rw * (d.beta_k_init != 0.0) +
+            I.io_bytes = 12.0 * (double)ncontrib + 12.0 * (double)nfcontrib + 8.0 * (double)nf * rw * (d.beta_k_init != 0.0) +
                          8.0 * ((double)nf * rw + 1) + 8.0 * 14.0 * nf;
         }
         I.rec_off = h->n_rec_total;
@@ -1345,11 +1304,10 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     h->dense_total = dense_off;
     if (h->elem_smem > 200 * 1024) return bail(fail(STRUT_UNSUPPORTED, "element fiber history exceeds shared memory"));
     h->elem_smem = std::max<size_t>(h->elem_smem, 16);
-    CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     if ((rc = elem_grid_of(h)) != STRUT_OK) return bail(rc);
     CK(cudaFuncSetAttribute(instance_newton_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)std::max<size_t>(h->inst_smem, 16)));
-    auto& al = h->allocs;
+    Arena& al = h->mem;
     // geometry and definitions
     DevMat* d_mats;
     DevSection* d_secs;
@@ -1410,49 +1368,16 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         const long long s2n = round4((int)std::max<long long>(s2_total, 4));
         const long long s1n = round4((int)std::max<long long>(s1_total, 4));
         const long long c1n = round4((int)std::max<long long>(c1_total, 4));
-        std::vector<double> c2(5 * c2n, 0.0), s2(10 * s2n, 0.0), s1(5 * s1n, 0.0), c1(6 * c1n, 0.0);
-        std::vector<int> kon(s2n, 0);
-        for (const DevElem& E : elems) {
-            const DevSection& sd = sp.secs[E.sec];
-            for (int ip = 0; ip < E.nip; ++ip) {
-                int base = sd.geo_off;
-                for (int j = 0; j < sd.n_s2; ++j) {
-                    const DevMat& m = mats[sp.m[base + j]];
-                    const long long idx = E.s2_off + ip * sd.n_s2 + j;
-                    s2[2 * s2n + idx] = m.p[1];
-                    s2[4 * s2n + idx] = m.k[S2K_EPSY];
-                    s2[3 * s2n + idx] = -m.k[S2K_EPSY];
-                    if (m.p[10] != 0.0) {
-                        s2[0 * s2n + idx] = m.k[S2K_SIGINI_E0];
-                        s2[1 * s2n + idx] = m.p[10];
-                    }
-                }
-                base += sd.n_s2;
-                for (int j = 0; j < sd.n_c2; ++j) {
-                    const DevMat& m = mats[sp.m[base + j]];
-                    c2[2 * c2n + E.c2_off + ip * sd.n_c2 + j] = m.k[C2K_EC0];
-                }
-                base += sd.n_c2;
-                for (int j = 0; j < sd.n_s1; ++j) {
-                    const DevMat& m = mats[sp.m[base + j]];
-                    s1[2 * s1n + E.s1_off + ip * sd.n_s1 + j] = m.p[1];
-                }
-                base += sd.n_s1;
-                for (int j = 0; j < sd.n_c1; ++j) {
-                    const DevMat& m = mats[sp.m[base + j]];
-                    c1[2 * c1n + E.c1_off + ip * sd.n_c1 + j] = m.k[C1K_EC0];
-                    c1[5 * c1n + E.c1_off + ip * sd.n_c1 + j] = m.k[C1K_EC0];
-                }
-            }
-        }
-        if ((rc = upload(&h->fs.c2, c2, al)) || (rc = upload(&h->fs.s2, s2, al)) ||
-            (rc = upload(&h->fs.s2_kon, kon, al)) || (rc = upload(&h->fs.s1, s1, al)) ||
-            (rc = upload(&h->fs.c1, c1, al)))
+        if ((rc = dzeros(&h->fs.c2, (size_t)(5 * c2n), al)) || (rc = dzeros(&h->fs.s2, (size_t)(10 * s2n), al)) ||
+            (rc = dzeros(&h->fs.s2_kon, (size_t)s2n, al)) || (rc = dzeros(&h->fs.s1, (size_t)(5 * s1n), al)) ||
+            (rc = dzeros(&h->fs.c1, (size_t)(6 * c1n), al)))
             return bail(rc);
         h->fs.c2_n = c2n;
         h->fs.s2_n = s2n;
         h->fs.s1_n = s1n;
         h->fs.c1_n = c1n;
+        init_history_kernel<<<h->n_elem, 128, 0, h->stream>>>(h->d_elems, h->geo, h->fs);
+        CK(cudaGetLastError());
     }
     InstArrays& A = h->A;
     std::memset(&A, 0, sizeof(A));
@@ -1570,7 +1495,8 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             return bail(rc);
         {
             const int polls = kBarrierPolls;
-            CK(cudaMemcpy((char*)h->d_gb + offsetof(GridBarrier, limit), &polls, sizeof(int), cudaMemcpyHostToDevice));
+            CK(cudaMemcpyAsync((char*)h->d_gb + offsetof(GridBarrier, limit), &polls, sizeof(int),
+                               cudaMemcpyHostToDevice, h->stream));
         }
         h->lfactor_wide = h->max_large_bw > kLargeMaxBw ? 1 : 0;
         const void* fk = h->lfactor_wide ? (const void*)large_factor_kernel<kPanelWide, kLargeThreadsWide>
@@ -1589,7 +1515,6 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         CK(cudaFuncSetAttribute(large_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)large_solve_smem(h->max_large_n)));
     }
-    CK(cudaMallocHost((void**)&h->h_ctrl, 4 * sizeof(int)));
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
     std::memset(&h->P, 0, sizeof(h->P));
@@ -1597,7 +1522,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     // for betaKInit; the trial fiber state it produces is discarded (revert) by construction.
     {
         std::vector<int> ones(h->n_inst, 1);
-        CK(cudaMemcpy(A.active, ones.data(), sizeof(int) * h->n_inst, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(A.active, ones.data(), sizeof(int) * h->n_inst, cudaMemcpyHostToDevice, h->stream));
         if (!h->shells_h.empty()) {
             h->n_shells = (int)h->shells_h.size();
             int* d_err = nullptr;
@@ -1655,9 +1580,9 @@ int strut_gpu_run_steps(StrutHandle* h, int32_t n_steps, StrutStepStats* stats) 
     TRY(ensure_history(h, h->steps_done + n_steps));
     // ground accelerations of every step of this call: per instance 2 values + 2 flags
     if (h->ag_cap < n_steps) {
-        if (h->d_ag) cudaFree(h->d_ag);
+        if (h->d_ag) CK(cudaFreeAsync(h->d_ag, h->stream));
         h->d_ag = nullptr;
-        CK(cudaMalloc((void**)&h->d_ag, (size_t)n_steps * 4 * h->n_inst * sizeof(double)));
+        TRY(pool_alloc((void**)&h->d_ag, (size_t)n_steps * 4 * h->n_inst * sizeof(double), h->stream));
         h->ag_cap = n_steps;
     }
     {
@@ -1742,9 +1667,10 @@ int strut_gpu_run_steps(StrutHandle* h, int32_t n_steps, StrutStepStats* stats) 
                 TRY(launch_instances(h, INST_MODE_NEWTON, step));
                 newton_check_kernel<<<1, 32, 0, h->stream>>>(h->d_ctl, h->A.nactive, none, 0);
                 CK(cudaGetLastError());
-                CK(cudaMemcpyAsync(h->h_ctrl, h->A.nactive, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+                int n_act = 0;
+                CK(cudaMemcpyAsync(&n_act, h->A.nactive, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
                 CK(cudaStreamSynchronize(h->stream));
-                if (h->h_ctrl[0] <= 0) break;
+                if (n_act <= 0) break;
             }
             TRY(prof_begin(h));
             commit_kernel_of(h)<<<h->n_elem, commit_block(h), 0, h->stream>>>(
@@ -2100,7 +2026,7 @@ int strut_gpu_revert(StrutHandle* h) {
 // ---------------------------------------------------------------------------------------
 struct StrutSectionBatch {
     int n_inst = 0;
-    std::vector<void*> allocs;
+    Arena mem;  // on the legacy default stream
     Geo geo;
     DevSection sd;
     BatchState bs;  // bs.n_inst: allocated instances (a whole number of tiles), the field stride
@@ -2112,9 +2038,7 @@ struct StrutSectionBatch {
     int grid = 0;
     size_t smem = 0;
     int* d_err = nullptr;
-    ~StrutSectionBatch() {
-        for (void* p : allocs) cudaFree(p);
-    }
+    ~StrutSectionBatch() { mem.release(); }
 };
 
 extern "C" {
@@ -2125,56 +2049,39 @@ int strut_gpu_material_path(const StrutUniMaterial* material, const double* stra
     if (n == 0) return STRUT_OK;
     DevMat m = make_devmat(*material);
     double *d_s = nullptr, *d_o = nullptr;
-    CK(cudaMalloc((void**)&d_s, n * sizeof(double)));
-    CK(cudaMalloc((void**)&d_o, 2 * n * sizeof(double)));
+    TRY(pool_alloc((void**)&d_s, n * sizeof(double), nullptr));
+    TRY(pool_alloc((void**)&d_o, 2 * n * sizeof(double), nullptr));
     CK(cudaMemcpy(d_s, strains, n * sizeof(double), cudaMemcpyHostToDevice));
     material_path_kernel<<<1, 32>>>(m, d_s, n, d_o);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(out, d_o, 2 * n * sizeof(double), cudaMemcpyDeviceToHost);
-    cudaFree(d_s);
-    cudaFree(d_o);
+    cudaFreeAsync(d_s, nullptr);
+    cudaFreeAsync(d_o, nullptr);
     if (e != cudaSuccess) return fail(STRUT_CUDA_ERROR, cudaGetErrorString(e));
     return STRUT_OK;
 }
 
 }  // extern "C"
 
-// Initial committed state (UniMaterialState(mat_def), core.mojo:203-263) of n_inst copies of
-// the section sp.secs[0], laid out as section_batch_kernel reads it.
-static void batch_initial_state(const SectionPack& sp, const std::vector<DevMat>& mats, long long n_inst,
-                                std::vector<double>& s2, std::vector<double>& c2, std::vector<double>& s1,
-                                std::vector<double>& c1, std::vector<int>& kon) {
+// Arrays of bs.n_inst copies of the section sp.secs[0] in their initial committed state.
+static int batch_history(const SectionPack& sp, const Geo& g, BatchState& bs, Arena& al) {
     const DevSection& sd = sp.secs[0];
-    const int P2 = fs_pad4(sd.n_s2), P3 = fs_pad4(sd.n_c2), P1 = fs_pad4(sd.n_s1), P4 = fs_pad4(sd.n_c1);
-    const long long n2 = n_inst * P2, n3 = n_inst * P3, n1 = n_inst * P1, n4 = n_inst * P4;
-    s2.assign(10 * std::max<long long>(n2, 1), 0.0);
-    c2.assign(5 * std::max<long long>(n3, 1), 0.0);
-    s1.assign(5 * std::max<long long>(n1, 1), 0.0);
-    c1.assign(6 * std::max<long long>(n4, 1), 0.0);
-    kon.assign(std::max<long long>(n2, 1), 0);
-    for (long long i = 0; i < n_inst; ++i) {
-        int base = sd.geo_off;
-        for (int j = 0; j < sd.n_s2; ++j) {
-            const DevMat& m = mats[sp.m[base + j]];
-            const long long idx = i * P2 + j;
-            s2[2 * n2 + idx] = m.p[1];
-            s2[4 * n2 + idx] = m.k[S2K_EPSY];
-            s2[3 * n2 + idx] = -m.k[S2K_EPSY];
-            if (m.p[10] != 0.0) {
-                s2[idx] = m.k[S2K_SIGINI_E0];
-                s2[n2 + idx] = m.p[10];
-            }
-        }
-        base += sd.n_s2;
-        for (int j = 0; j < sd.n_c2; ++j) c2[2 * n3 + i * P3 + j] = mats[sp.m[base + j]].k[C2K_EC0];
-        base += sd.n_c2;
-        for (int j = 0; j < sd.n_s1; ++j) s1[2 * n1 + i * P1 + j] = mats[sp.m[base + j]].p[1];
-        base += sd.n_s1;
-        for (int j = 0; j < sd.n_c1; ++j) {
-            c1[2 * n4 + i * P4 + j] = mats[sp.m[base + j]].k[C1K_EC0];
-            c1[5 * n4 + i * P4 + j] = mats[sp.m[base + j]].k[C1K_EC0];
-        }
+    bs.p_s2 = fs_pad4(sd.n_s2);
+    bs.p_c2 = fs_pad4(sd.n_c2);
+    bs.p_s1 = fs_pad4(sd.n_s1);
+    bs.p_c1 = fs_pad4(sd.n_c1);
+    const size_t n = (size_t)bs.n_inst;
+    TRY(dzeros(&bs.s2, 10 * n * bs.p_s2, al));
+    TRY(dzeros(&bs.c2, 5 * n * bs.p_c2, al));
+    TRY(dzeros(&bs.s1, 5 * n * bs.p_s1, al));
+    TRY(dzeros(&bs.c1, 6 * n * bs.p_c1, al));
+    TRY(dzeros(&bs.kon, n * bs.p_s2, al));
+    const long long t = bs.n_inst * (sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1);
+    if (t > 0) {
+        init_batch_kernel<<<(unsigned)((t + 255) / 256), 256, 0, al.s>>>(g, sd, bs);
+        CK(cudaGetLastError());
     }
+    return STRUT_OK;
 }
 
 // Persistent grid of the streaming kernel: as many CTAs per SM as the occupancy calculator
@@ -2218,7 +2125,7 @@ int strut_gpu_section_batch_create(const StrutUniMaterial* materials, int32_t nu
     DevSection* d_secs;
     double *d_y, *d_a;
     int* d_m;
-    auto& al = b->allocs;
+    Arena& al = b->mem;
     if ((rc = upload(&d_mats, mats, al)) || (rc = upload(&d_secs, sp.secs, al)) || (rc = upload(&d_y, sp.y, al)) ||
         (rc = upload(&d_a, sp.a, al)) || (rc = upload(&d_m, sp.m, al))) {
         delete b;
@@ -2229,27 +2136,19 @@ int strut_gpu_section_batch_create(const StrutUniMaterial* materials, int32_t nu
     b->geo.m = d_m;
     b->geo.mats = d_mats;
     b->geo.secs = d_secs;
-    std::vector<double> s2, c2, s1, c1;
-    std::vector<int> kon;
     if ((rc = fs_configure(b)) != STRUT_OK) {
         delete b;
         return rc;
     }
-    const long long n_alloc = b->n_tiles * kFsTile;  // whole tiles: a tile's copies stay in bounds
-    batch_initial_state(sp, mats, n_alloc, s2, c2, s1, c1, kon);
-    if ((rc = upload(&b->bs.s2, s2, al)) || (rc = upload(&b->bs.c2, c2, al)) || (rc = upload(&b->bs.s1, s1, al)) ||
-        (rc = upload(&b->bs.c1, c1, al)) || (rc = upload(&b->bs.kon, kon, al))) {
+    b->bs.n_inst = b->n_tiles * kFsTile;  // whole tiles: a tile's copies stay in bounds
+    if ((rc = batch_history(sp, b->geo, b->bs, al)) || (rc = dzeros(&b->d_err, 1, al))) {
         delete b;
         return rc;
     }
-    b->bs.n_inst = n_alloc;
-    b->bs.p_s2 = b->L.p_s2;
-    b->bs.p_c2 = b->L.p_c2;
-    b->bs.p_s1 = b->L.p_s1;
-    b->bs.p_c1 = b->L.p_c1;
-    if ((rc = dzeros(&b->d_err, 1, al))) {
+    // the caller evaluates on streams of its own
+    if (cudaStreamSynchronize(al.s) != cudaSuccess) {
         delete b;
-        return rc;
+        return fail(STRUT_CUDA_ERROR, "section batch initialisation failed");
     }
     *out = b;
     return STRUT_OK;
@@ -2327,8 +2226,9 @@ int strut_gpu_section_path(const StrutUniMaterial* materials, int32_t num_materi
     int rc = strut_gpu_section_batch_create(materials, num_materials, fibers, num_fibers, 1, &b);
     if (rc != STRUT_OK) return rc;
     double *d_ek = nullptr, *d_r = nullptr;
-    cudaError_t e = cudaMalloc((void**)&d_ek, 2 * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_r, 5 * sizeof(double));
+    cudaError_t e = cudaSuccess;
+    if ((rc = pool_alloc((void**)&d_ek, 2 * sizeof(double), nullptr)) == STRUT_OK)
+        rc = pool_alloc((void**)&d_r, 5 * sizeof(double), nullptr);
     for (int p = 0; p < n_points && e == cudaSuccess && rc == STRUT_OK; ++p) {
         e = cudaMemcpy(d_ek, eps0_kappa + 2 * p, 2 * sizeof(double), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) break;
@@ -2336,8 +2236,8 @@ int strut_gpu_section_path(const StrutUniMaterial* materials, int32_t num_materi
         if (rc != STRUT_OK) break;
         e = cudaMemcpy(out + 5 * p, d_r, 5 * sizeof(double), cudaMemcpyDeviceToHost);
     }
-    if (d_ek) cudaFree(d_ek);
-    if (d_r) cudaFree(d_r);
+    if (d_ek) cudaFreeAsync(d_ek, nullptr);
+    if (d_r) cudaFreeAsync(d_r, nullptr);
     strut_gpu_section_batch_destroy(b);
     if (e != cudaSuccess) return fail(STRUT_CUDA_ERROR, cudaGetErrorString(e));
     return rc;
@@ -2354,13 +2254,8 @@ int strut_gpu_section3d_path(const StrutUniMaterial* materials, int32_t num_mate
     if (n_points == 0) return STRUT_OK;
     std::vector<DevMat> mats;
     for (int i = 0; i < num_materials; ++i) mats.push_back(make_devmat(materials[i]));
-    std::vector<double> s2, c2, s1, c1;
-    std::vector<int> kon;
-    batch_initial_state(sp, mats, 1, s2, c2, s1, c1, kon);
-    std::vector<void*> al;
-    auto cleanup = [&]() {
-        for (void* p : al) cudaFree(p);
-    };
+    Arena al;
+    auto cleanup = [&]() { al.release(); };
     DevMat* d_mats = nullptr;
     double *d_y = nullptr, *d_z = nullptr, *d_a = nullptr, *d_path = nullptr, *d_out = nullptr;
     int* d_m = nullptr;
@@ -2368,18 +2263,10 @@ int strut_gpu_section3d_path(const StrutUniMaterial* materials, int32_t num_mate
     std::memset(&bs, 0, sizeof(bs));
     std::vector<double> pv(path, path + 3 * (size_t)n_points);
     if ((rc = upload(&d_mats, mats, al)) || (rc = upload(&d_y, sp.y, al)) || (rc = upload(&d_z, sp.z, al)) ||
-        (rc = upload(&d_a, sp.a, al)) || (rc = upload(&d_m, sp.m, al)) || (rc = upload(&bs.s2, s2, al)) ||
-        (rc = upload(&bs.c2, c2, al)) || (rc = upload(&bs.s1, s1, al)) || (rc = upload(&bs.c1, c1, al)) ||
-        (rc = upload(&bs.kon, kon, al)) ||
-        (rc = upload(&d_path, pv, al)) || (rc = dzeros(&d_out, 9 * (size_t)n_points, al))) {
+        (rc = upload(&d_a, sp.a, al)) || (rc = upload(&d_m, sp.m, al)) || (rc = upload(&d_path, pv, al)) || (rc = dzeros(&d_out, 9 * (size_t)n_points, al))) {
         cleanup();
         return rc;
     }
-    bs.n_inst = 1;
-    bs.p_s2 = fs_pad4(sp.secs[0].n_s2);
-    bs.p_c2 = fs_pad4(sp.secs[0].n_c2);
-    bs.p_s1 = fs_pad4(sp.secs[0].n_s1);
-    bs.p_c1 = fs_pad4(sp.secs[0].n_c1);
     Geo g;
     std::memset(&g, 0, sizeof(g));
     g.y = d_y;
@@ -2387,6 +2274,11 @@ int strut_gpu_section3d_path(const StrutUniMaterial* materials, int32_t num_mate
     g.a = d_a;
     g.m = d_m;
     g.mats = d_mats;
+    bs.n_inst = 1;
+    if ((rc = batch_history(sp, g, bs, al)) != STRUT_OK) {
+        cleanup();
+        return rc;
+    }
     section3d_path_kernel<<<1, 32>>>(g, sp.secs[0], bs, d_path, n_points, d_out);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(out, d_out, 9 * (size_t)n_points * sizeof(double), cudaMemcpyDeviceToHost);
