@@ -18,6 +18,7 @@
 //   tests                     nonlinear_convergence.mojo:8-20, transient_nonlinear.mojo:2798-2811
 #pragma once
 
+#include "band_pivot.cuh"
 #include "band_warp.cuh"
 #include "kernels.cuh"
 
@@ -535,6 +536,11 @@ __device__ void dense_solve_warp(const double* D, const int* piv, int n, const d
 __device__ void newton_tail(const DevInst& I, InstArrays& A, int inst, const double* du,
                             const double* R, int* hrow, double* red, int* red_r);
 
+// PIVOT: the instance for 3D handles, whose systems with rigid diaphragms need row interchanges in
+// every factorisation; they run band_pivot_solve (band_pivot.cuh).  Its registers would keep two 2D
+// instances from sharing an SM, and a 2D frame's system needs an interchange once in some thousand
+// factorisations: 2D handles keep the dense LU for it, results included.
+template <bool PIVOT>
 __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __restrict__ insts,
                                                               InstArrays A0, int mode, int step) {
     InstArrays A = A0;
@@ -545,6 +551,7 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
     __shared__ int s_it;  // this instance's Newton iterations of the step so far
     __shared__ double s_rk[2], s_z[2];  // band_lu_cta
     __shared__ int s_flag[2];
+    __shared__ __align__(16) double s_pbuf[PIVOT ? kPivotBuf : 2];
     const int inst = blockIdx.x;
     const int tid = threadIdx.x, nt = blockDim.x;
     {
@@ -762,7 +769,13 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
     double* D = A.dense + I.dense_off;
     int* piv = A.piv + f0;
     bool forward = false;  // w holds L^-1 R already
-    if (!refresh) {
+    // an instance that has needed interchanges before goes straight to the pivoted factorisation,
+    // which makes none where none is needed
+    const bool can_pivot = PIVOT && refresh && !modified && !I.spd && bw <= kPivotMaxBw;
+    bool pivoted = can_pivot && A.fallbacks && A.fallbacks[inst] > 0;
+    int swaps = 0;
+    if (pivoted) {
+    } else if (!refresh) {
         // the step's factors
         dense = A.lu_dense[inst] != 0;
         if (!dense) {
@@ -781,6 +794,24 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
         forward = true;
     } else {
         rc = band_lu_smem(Kb, n, bw, rw, fac);
+    }
+    if (can_pivot && (pivoted || rc == 6)) {
+        __syncthreads();
+        if (!pivoted) {
+            // the assembled values again
+            const double* Kinit = A.Kinit + I.band_off;
+            for (int t = tid; t < n * rw; t += nt) {
+                const int i = t / rw, j = i + t % rw - bw;
+                if (j < 0 || j >= n) continue;
+                Kb[t] = mode == INST_MODE_SOLVE_EXPORTED ? A.export_band[I.band_off + t]
+                                                         : keff_slot(I, A, I.slot_ptr_off, Kinit, i, j, t);
+            }
+            pivoted = true;
+        }
+        for (int i = tid; i < n; i += nt) w[i] = R[i];
+        __syncthreads();
+        rc = band_pivot_solve(Kb, n, bw, rw, w, du, D, s_pbuf, &swaps);
+        if (tid == 0 && swaps > 0 && A.fallbacks) A.fallbacks[inst] += 1;
     }
     if (refresh && rc == 6) {
         // BandGeneral: a row swap would be needed, so the whole effective matrix is factored
@@ -829,7 +860,9 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
     // multipliers of the last column were written in the loop except column n-1 (none below)
     __syncthreads();
     if (tid < 32) {
-        if (dense)
+        if (pivoted)
+            ;  // solved with the factorisation
+        else if (dense)
             dense_solve_warp(D, piv, n, R, w, du);
         else if (I.spd)
             band_solve_chol_warp(Kb, n, bw, rw, R, w, du, fac);

@@ -397,6 +397,7 @@ static int prof_end(StrutHandle* h, int k) {
 // threads per integration point up to 5 points, else 64.
 using CommitKernel = decltype(&commit_kernel<128>);
 using ElemKernel = decltype(&element_state_kernel<2>);
+using InstKernel = decltype(&instance_newton_kernel<false>);
 // Element CTA sizes: 640 (one CTA per SM), 320, 224 and 160 threads (more CTAs per SM where
 // shared memory allows: more elements in flight, each with fewer threads).  The 3D kernel's
 // epilogue needs 172 threads, so 160 is 2D only.
@@ -409,6 +410,9 @@ static int elem_threads_of(const StrutHandle* h) {
 }
 static ElemKernel elem_kernel_of(const StrutHandle* h) {
     return h->ndf_all == 6 ? element_state_kernel<3> : element_state_kernel<2>;
+}
+static InstKernel inst_kernel_of(const StrutHandle* h) {
+    return h->ndf_all == 6 ? instance_newton_kernel<true> : instance_newton_kernel<false>;
 }
 static dim3 elem_block(const StrutHandle* h) { return dim3(elem_threads_of(h)); }
 // Resident CTAs of the element kernel the handle's tuning selects (its persistent grid).
@@ -531,7 +535,7 @@ static int launch_instances(StrutHandle* h, int mode, int step) {
     A.hist_iters = (mode == INST_MODE_NEWTON && step >= 0) ? h->d_hist_iters : nullptr;
     A.bytes_counter = h->d_counters + 4;
     TRY(prof_begin(h));
-    instance_newton_kernel<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, mode, step);
+    inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, mode, step);
     CK(cudaGetLastError());
     TRY(launch_large(h, mode, nullptr, &A));
     TRY(prof_end(h, 1));
@@ -681,7 +685,7 @@ static int build_graph(StrutHandle* h) {
                             (const double*)h->A.u_full));
         n_after_el = n_sh;
     }
-    TRY(add_kernel_node(&n_in, ibody, &n_after_el, 1, instance_newton_kernel, dim3(h->n_inst), dim3(256),
+    TRY(add_kernel_node(&n_in, ibody, &n_after_el, 1, inst_kernel_of(h), dim3(h->n_inst), dim3(256),
                         h->inst_smem, (const DevInst*)h->d_insts, A, (int)INST_MODE_NEWTON, 0));
     cudaGraphNode_t n_before_chk = n_in;
     TRY(add_kernel_node(&n_chk, ibody, &n_before_chk, 1, newton_check_kernel, dim3(1), dim3(32), 0, h->d_ctl,
@@ -1169,7 +1173,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         I.slot_ptr_off = band_off;
         I.dense_off = dense_off;
         if ((size_t)nf * rw * sizeof(double) + 6 * sizeof(double) * (size_t)nf <= 220 * 1024)
-            dense_off += (long long)nf * nf;
+            dense_off += (long long)nf * std::max(nf, rw);  // dense LU, or the pivoted band's U
         I.elem_off = e0;
         I.n_elem = d.num_elements;
         I.fint_ptr_off = f_off;
@@ -1305,7 +1309,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     if (h->elem_smem > 200 * 1024) return bail(fail(STRUT_UNSUPPORTED, "element fiber history exceeds shared memory"));
     h->elem_smem = std::max<size_t>(h->elem_smem, 16);
     if ((rc = elem_grid_of(h)) != STRUT_OK) return bail(rc);
-    CK(cudaFuncSetAttribute(instance_newton_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CK(cudaFuncSetAttribute(inst_kernel_of(h), cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)std::max<size_t>(h->inst_smem, 16)));
     Arena& al = h->mem;
     // geometry and definitions
@@ -1549,7 +1553,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         if ((rc = upload(&d_tmp, tmp, al))) return bail(rc);
         InstArrays B = A;
         B.export_band = d_Kinit;
-        instance_newton_kernel<<<h->n_inst, 256, h->inst_smem, h->stream>>>(d_tmp, B, INST_MODE_EXPORT, -1);
+        inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(d_tmp, B, INST_MODE_EXPORT, -1);
         CK(cudaGetLastError());
         if ((rc = launch_large(h, INST_MODE_EXPORT, d_tmp, &B)) != STRUT_OK) return bail(rc);
         CK(cudaStreamSynchronize(h->stream));
@@ -1990,7 +1994,7 @@ int strut_gpu_factor_solve(StrutHandle* h, const double* rhs, double* du) {
     A.rhs_in = h->d_rhs;
     std::vector<int> zeros(h->n_inst, 0);
     CK(cudaMemcpyAsync(h->A.status, zeros.data(), sizeof(int) * h->n_inst, cudaMemcpyHostToDevice, h->stream));
-    instance_newton_kernel<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, INST_MODE_SOLVE_EXPORTED, -1);
+    inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, INST_MODE_SOLVE_EXPORTED, -1);
     CK(cudaGetLastError());
     TRY(launch_large(h, INST_MODE_SOLVE_EXPORTED, nullptr, &A));
     CK(cudaStreamSynchronize(h->stream));
