@@ -32,7 +32,7 @@ constexpr int kPivotBuf = 64 * (2 + kPivotThreads / 32);  // doubles of shared m
 // memory) to L^-1 P w; U(k, j) to U[k * rw + j - k].  buf: kPivotBuf doubles of shared memory, 16-byte
 // aligned.  Returns 0, 2 (singular) on every thread; *swaps counts the interchanges.
 template <int R>
-__device__ __noinline__ int band_lu_pivot(const double* Kb, int n, int bw, int rw, double* w, double* U, double* buf,
+__device__ __forceinline__ int band_lu_pivot(const double* Kb, int n, int bw, int rw, double* w, double* U, double* buf,
                                           int* swaps) {
     constexpr unsigned all = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -141,7 +141,7 @@ __device__ __noinline__ int band_lu_pivot(const double* Kb, int n, int bw, int r
 // U x = w (U as band_lu_pivot leaves it) in blocks of 32 rows from the end: the warps form the
 // rows' sums over the columns behind the block, the first warp solves the block's triangle.  Us:
 // n x rw doubles of shared memory for U, t: 32 doubles.
-__device__ __noinline__ void band_pivot_back(const double* U, double* Us, int n, int bw, int rw, const double* w,
+__device__ __forceinline__ void band_pivot_back(const double* U, double* Us, int n, int bw, int rw, const double* w,
                                              double* x, double* t) {
     constexpr unsigned all = 0xffffffffu;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
@@ -182,7 +182,7 @@ __device__ __noinline__ void band_pivot_back(const double* U, double* Us, int n,
 __device__ __forceinline__ int band_pivot_solve(double* Kb, int n, int bw, int rw, double* w, double* x, double* U,
                                                 double* buf, int* swaps) {
     const int rc = bw < 32   ? band_lu_pivot<32>(Kb, n, bw, rw, w, U, buf, swaps)
-                   : bw < 56 ? band_lu_pivot<56>(Kb, n, bw, rw, w, U, buf, swaps)
+                   : bw < 58 ? band_lu_pivot<58>(Kb, n, bw, rw, w, U, buf, swaps)
                              : band_lu_pivot<64>(Kb, n, bw, rw, w, U, buf, swaps);
     if (rc != 0) return rc;
     band_pivot_back(U, Kb, n, bw, rw, w, x, buf);

@@ -1,7 +1,7 @@
 // Newton iteration of instances whose effective band does not fit in shared memory (a 3D frame
 // of a few thousand dofs and a bandwidth of a few hundred: ~10-30 MB, resident in the 126 MB L2).
 //
-//   large_assemble_kernel  one warp per band row: K gathered per slot in element order, C, the
+//   large_assemble_kernel  one warp per band row: K of gather_kernel, C, the
 //                          effective entries K + a1 C + a0 M written to the global band, the row's
 //                          residual P - F_int - C v - M a (transient_nonlinear.mojo:2302-2356,
 //                          linear_solver_backend.mojo:1877-1983)
@@ -124,7 +124,6 @@ __global__ void __launch_bounds__(256) large_assemble_kernel(const DevInst* __re
         A.iters[inst] += 1;
         if (A.bytes_counter) atomicAdd(A.bytes_counter, (unsigned long long)I.io_bytes);
     }
-    const long long sp0 = I.slot_ptr_off;
     const double* Kinit = A.Kinit + I.band_off;
     double* B = A.lband + I.lband_off + (long long)i * I.lrw;
     for (int o = rw + lane; o < I.lrw; o += 32) B[o] = 0.0;  // fill slots
@@ -137,7 +136,7 @@ __global__ void __launch_bounds__(256) large_assemble_kernel(const DevInst* __re
             if (mode == INST_MODE_EXPORT) A.export_band[I.band_off + slot] = 0.0;
             continue;
         }
-        const double K = gather_slot(A, sp0, (int)slot);
+        const double K = A.kband[I.band_off + slot];
         double C = 0.0;
         if (I.has_damping) {
             C = I.alpha_m * (i == j ? A.Mrff[f0 + i] : 0.0);
@@ -158,8 +157,7 @@ __global__ void __launch_bounds__(256) large_assemble_kernel(const DevInst* __re
     if (lane == 0) {
         const int gi = f0 + i;
         const double an = I.a0 * (A.u_f[gi] - A.u_n[gi]) - I.a2 * A.v_n[gi] - I.a3 * A.a_n[gi];
-        const int q0 = A.fint_ptr[I.fint_ptr_off + i], q1 = A.fint_ptr[I.fint_ptr_off + i + 1];
-        const double F = gather_fint(A, A.ef, q0, q1);
+        const double F = A.fsum[gi];
         const double ma = A.Mff[gi] * an;
         A.R[gi] = A.P_f[gi] - F - 0.0 - cv - ma;
         wbuf[gi] = A.R[gi];

@@ -29,6 +29,7 @@
 #include "fiber_stream_kernels.cuh"
 #include "init_kernels.cuh"
 #include "solver_kernels.cuh"
+#include "gather_kernels.cuh"
 #include "largeband_kernels.cuh"
 #include "shell_kernels.cuh"
 #include "predictor_kernels.cuh"
@@ -281,6 +282,9 @@ struct StrutHandle {
     std::vector<int> sec_off, sec_n;
     double* d_hist_sec = nullptr;
     long long ek_total = 0, ef_total = 0;
+    // 3D: assembled K and F_int (gather_kernel) and its grid
+    double *d_kband = nullptr, *d_fsum = nullptr;
+    int gather_slot_blocks = 0, gather_dof_blocks = 0;
     std::vector<DevShell> shells_h;  // linear shells of all instances
     DevShell* d_shells = nullptr;
     int n_shells = 0;
@@ -530,11 +534,24 @@ static int launch_large(StrutHandle* h, int mode, const DevInst* insts = nullptr
     return STRUT_OK;
 }
 
+// Assembly of a 3D handle's instances (gather_kernel) before the instance kernels that read it.
+static dim3 gather_grid(const StrutHandle* h) {
+    return dim3(h->gather_slot_blocks + h->gather_dof_blocks, h->n_inst);
+}
+static int launch_gather(StrutHandle* h, const DevInst* insts, int mode) {
+    if (!h->d_kband || mode == INST_MODE_SOLVE_EXPORTED) return STRUT_OK;
+    gather_kernel<<<gather_grid(h), 256, 0, h->stream>>>(insts, h->A, mode == INST_MODE_NEWTON ? 1 : 0,
+                                                         h->gather_slot_blocks, h->d_kband, h->d_fsum);
+    CK(cudaGetLastError());
+    return STRUT_OK;
+}
+
 static int launch_instances(StrutHandle* h, int mode, int step) {
     InstArrays A = h->A;
     A.hist_iters = (mode == INST_MODE_NEWTON && step >= 0) ? h->d_hist_iters : nullptr;
     A.bytes_counter = h->d_counters + 4;
     TRY(prof_begin(h));
+    TRY(launch_gather(h, h->d_insts, mode));
     inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, mode, step);
     CK(cudaGetLastError());
     TRY(launch_large(h, mode, nullptr, &A));
@@ -685,6 +702,12 @@ static int build_graph(StrutHandle* h) {
                             (const double*)h->A.u_full));
         n_after_el = n_sh;
     }
+    if (h->d_kband) {
+        cudaGraphNode_t n_g;
+        TRY(add_kernel_node(&n_g, ibody, &n_after_el, 1, gather_kernel, gather_grid(h), dim3(256), 0,
+                            (const DevInst*)h->d_insts, A, 1, h->gather_slot_blocks, h->d_kband, h->d_fsum));
+        n_after_el = n_g;
+    }
     TRY(add_kernel_node(&n_in, ibody, &n_after_el, 1, inst_kernel_of(h), dim3(h->n_inst), dim3(256),
                         h->inst_smem, (const DevInst*)h->d_insts, A, (int)INST_MODE_NEWTON, 0));
     cudaGraphNode_t n_before_chk = n_in;
@@ -775,6 +798,10 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     std::vector<double> slot_coef, fint_coef;        // filled when some instance has constraints
     std::vector<int> sl_dof, sl_ptr(1, 0), sl_master;
     std::vector<double> sl_coef;
+    std::vector<int8_t> efree8;  // 2D: free dofs of each element (InstArrays::efree)
+    std::vector<int> efirst;
+    bool efree_ok = true;  // they fit eight bits relative to the first
+    bool any_kinit = false;
     bool any_mpc = false;
     for (int inst = 0; inst < num_instances; ++inst) any_mpc = any_mpc || models[inst].num_slaves > 0;
     long long c2_total = 0, s2_total = 0, s1_total = 0, c1_total = 0;
@@ -1032,6 +1059,18 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
                 E.commit_bytes = 2.0 * fib + est + 8.0 * nd + (double)sizeof(DevElem);
             }
             elems.push_back(E);
+            if (!three_d) {
+                const int* fr = &efree[(size_t)nd * e];
+                int lo = -1;
+                for (int a = 0; a < 6; ++a)
+                    if (fr[a] >= 0 && (lo < 0 || fr[a] < lo)) lo = fr[a];
+                efirst.push_back(std::max(lo, 0));
+                for (int a = 0; a < 8; ++a) {
+                    const int rel = a < 6 && fr[a] >= 0 ? fr[a] - lo : -1;
+                    if (rel > 127) efree_ok = false;
+                    efree8.push_back((int8_t)(rel > 127 ? -1 : rel));
+                }
+            }
             for (int a = 0; a < nd; ++a) {
                 const int ia = efree[(size_t)nd * e + a];
                 if (ia < 0) continue;
@@ -1221,6 +1260,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             h->max_iters_global = std::max(h->max_iters_global, total);
         }
         I.spd = d.system == STRUT_SYSTEM_BAND_SPD;
+        any_kinit = any_kinit || d.beta_k_init != 0.0;
         I.has_damping = d.alpha_m != 0.0 || d.beta_k != 0.0 || d.beta_k_init != 0.0 || d.beta_k_comm != 0.0;
         I.dt = d.dt;
         I.gamma = d.gamma;
@@ -1481,6 +1521,25 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         std::vector<int> neg(h->n_inst, -1);
         if ((rc = upload(&h->d_fail_step, neg, al))) return bail(rc);
     }
+    if (h->ndf_all == 6) {
+        int slots = 0, dofs = 0;
+        for (const DevInst& I : h->insts) {
+            slots = std::max(slots, I.n * I.rw);
+            dofs = std::max(dofs, I.n);
+        }
+        h->gather_slot_blocks = (slots + 255) / 256;
+        h->gather_dof_blocks = (dofs + 255) / 256;
+        if ((rc = dzeros(&h->d_kband, (size_t)h->band_total, al)) || (rc = dzeros(&h->d_fsum, nF, al)))
+            return bail(rc);
+        A.kband = h->d_kband;
+        A.fsum = h->d_fsum;
+    } else if (!any_mpc && efree_ok) {
+        int8_t* d_ef;
+        int* d_e1;
+        if ((rc = upload(&d_ef, efree8, al)) || (rc = upload(&d_e1, efirst, al))) return bail(rc);
+        A.efree = d_ef;
+        A.efirst = d_e1;
+    }
     A.ctl = h->d_ctl;
     A.estate = h->d_estate;
     A.n_free_total = h->n_free_total;
@@ -1553,9 +1612,17 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         if ((rc = upload(&d_tmp, tmp, al))) return bail(rc);
         InstArrays B = A;
         B.export_band = d_Kinit;
+        if ((rc = launch_gather(h, d_tmp, INST_MODE_EXPORT)) != STRUT_OK) return bail(rc);
         inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(d_tmp, B, INST_MODE_EXPORT, -1);
         CK(cudaGetLastError());
         if ((rc = launch_large(h, INST_MODE_EXPORT, d_tmp, &B)) != STRUT_OK) return bail(rc);
+        if (any_kinit) {
+            double* kt = nullptr;
+            if ((rc = dzeros(&kt, (size_t)h->band_total, al)) != STRUT_OK) return bail(rc);
+            kinit_by_column_kernel<<<h->n_inst, 256, 0, h->stream>>>(h->d_insts, d_Kinit, kt);
+            CK(cudaGetLastError());
+            A.KinitT = kt;
+        }
         CK(cudaStreamSynchronize(h->stream));
         std::vector<int> st(h->n_inst);
         CK(cudaMemcpy(st.data(), A.status, sizeof(int) * h->n_inst, cudaMemcpyDeviceToHost));
