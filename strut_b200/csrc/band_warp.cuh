@@ -11,7 +11,7 @@
 // is chaotic at the rounding level, and one record of 256 ended elsewhere).
 #pragma once
 
-#include <cstdint>
+#include "quotient.cuh"
 
 namespace strut {
 
@@ -20,25 +20,6 @@ constexpr int kBackWarpMax = 24;   // widest half band of the one-warp back subs
 constexpr int kBackWarpGroup = 8;  // unknowns per window position
 constexpr int kLuRowsMax = 62;     // widest half band of band_lu_cta
 constexpr int kLuRowsThreads = 256;
-
-// v / d given r = 1 / d: the quotient by Markstein's correction (the residual v - q d is exact in a
-// fused multiply-add), equal to the correctly rounded quotient away from overflow and underflow.
-// A zero numerator, which is common in a band, costs an FP64 division 413 cycles instead of
-// 132 (measured, with the add behind it); here it costs what any other does.
-__device__ __forceinline__ double quot(double v, double d, double r) {
-    const double q = v * r;
-    return fma(fma(-q, d, v), r, q);
-}
-
-// 1 / d by Newton's method (third order: y (1 + e + e^2), e = 1 - d y) from the hardware's
-// approximation, for finite d away from underflow; within an ulp of the correctly rounded value.
-// Off the quotient's error: quot() corrects with the exact residual.
-__device__ __forceinline__ double recip(double d) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-d, y, 1.0);
-    return fma(fma(e, e, e), y, y);
-}
 
 // Barrier of the first nt threads of the CTA (a multiple of 32).
 __device__ __forceinline__ void bar_first(int nt) { asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory"); }
@@ -54,10 +35,12 @@ __device__ __forceinline__ void bar_first(int nt) { asm volatile("bar.sync 1, %0
 // next to it the instructions of a warp that works alone on its scheduler.  So the step has no
 // inner loop, no division (74 cycles, 413 with a zero numerator, which bands are full of; recip 40,
 // quot 24) and no reducing barrier (63 against 28 cycles): a row that needs an interchange raises a
-// flag that the next step reads with its other operands.  While all bw rows exist, every operand
+// flag that the next step reads with its other operands.  Flags alternate between two places by the
+// step's parity: a place is written in one step and read in the next only, so all warps leave the
+// loop at the same step.  While all bw rows exist, every operand
 // has a pointer that moves by a fixed stride; rows and columns that a warp or lane does not have
 // point at the zeros z (stride 0) instead of being tested.
-// NR NW >= bw, 32 NC > bw.  rk: 2 doubles; z: 2 doubles; flag: 2 ints of shared memory.  Returns
+// NR NW >= bw, 32 NC > bw.  rk: 2 doubles; z: 2 doubles; flag: 4 ints of shared memory.  Returns
 // 0 ok, 2 singular, 6 a row swap would be needed (the caller then starts again from the assembled
 // values), on the threads of the first NW warps.
 template <int NR, int NC, int NW, bool KEEP>
@@ -68,8 +51,10 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
     if (threadIdx.x == 0) {
         rk[0] = recip(B[bw]);
         z[0] = z[1] = 0.0;
-        flag[0] = flag[1] = 0;
+        flag[0] = flag[1] = flag[2] = flag[3] = 0;
     }
+    // what step k of an elimination that cannot go on means: a row swap (6) or a singular matrix
+    auto verdict = [&](int k) { return flag[2 * (k & 1)] && flag[2 * (k & 1) + 1] ? 6 : 2; };
     const double* pf[NR];  // B(i, k) of this warp's rows
     double* pa[NR][NC];    // this lane's entries of them
     const double* pu[NC];  // and of row k
@@ -96,7 +81,7 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
 #pragma unroll 1
     for (; k + bw < n; ++k) {
         const double akk = *pk, rkk = rk[k & 1], pa_ = fabs(akk);
-        const int failed = flag[0];
+        if (flag[2 * ((k + 1) & 1)]) return verdict(k - 1);  // raised in step k - 1
         double f[NR], uk[NC], a[NR][NC];
 #pragma unroll
         for (int u = 0; u < NR; ++u) f[u] = *pf[u];
@@ -124,19 +109,18 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
         if (swap) {
             // pivot search of linear_solver_backend.mojo:640-657: an entry strictly larger than
             // the diagonal selects another row; the largest one decides singularity
-            flag[0] = 1;
+            flag[2 * (k & 1)] = 1;
 #pragma unroll
             for (int u = 0; u < NR; ++u)
-                if (fabs(f[u]) > 1.0e-14) flag[1] = 1;
+                if (fabs(f[u]) > 1.0e-14) flag[2 * (k & 1) + 1] = 1;
         }
 #pragma unroll
         for (int v = 0; v < NC; ++v) pu[v] += su[v];
         pk += rw;
         bar_first(NT);
-        if (failed || pa_ <= 1.0e-14) break;
+        if (pa_ <= 1.0e-14) return verdict(k);
     }
-    if (flag[0]) return flag[1] ? 6 : 2;
-    if (k + bw < n) return 2;
+    if (k > 0 && flag[2 * ((k + 1) & 1)]) return verdict(k - 1);
     // the last bw columns, fewer rows and columns each
     int dk = k * rw + bw;
 #pragma unroll 1
@@ -171,15 +155,14 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
             if (KEEP && lane == 0) B[d] = q;
         }
         if (swap) {
-            flag[0] = 1;
+            flag[2 * (k & 1)] = 1;
 #pragma unroll
             for (int u = 0; u < NR; ++u)
-                if (1 + warp + NW * u <= m && fabs(f[u]) > 1.0e-14) flag[1] = 1;
+                if (1 + warp + NW * u <= m && fabs(f[u]) > 1.0e-14) flag[2 * (k & 1) + 1] = 1;
         }
         dk += rw;
         bar_first(NT);
-        if (flag[0]) return flag[1] ? 6 : 2;
-        if (pa_ <= 1.0e-14) return 2;
+        if (flag[2 * (k & 1)] || pa_ <= 1.0e-14) return verdict(k);
     }
     return 0;
 }

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
     __shared__ double red[32];
     __shared__ int red_r[32];
     __shared__ double s_rk[2], s_z[2];  // band_lu_cta
-    __shared__ int s_flag[2];
+    __shared__ int s_flag[4];
     const int tid = threadIdx.x, nt = blockDim.x;
     const int rw = 2 * bw + 1;
     double* Kb = smem_one;

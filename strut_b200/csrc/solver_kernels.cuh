@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(256) instance_newton_kernel(const DevInst* __r
     __shared__ int red_r[32];
     __shared__ int s_it;  // this instance's Newton iterations of the step so far
     __shared__ double s_rk[2], s_z[2];  // band_lu_cta
-    __shared__ int s_flag[2];
+    __shared__ int s_flag[4];
     __shared__ __align__(16) double s_pbuf[PIVOT ? kPivotBuf : 2];
     const int inst = blockIdx.x;
     const int tid = threadIdx.x, nt = blockDim.x;
