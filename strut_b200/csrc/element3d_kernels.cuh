@@ -82,7 +82,7 @@ __device__ __forceinline__ void fiber_phase3(const Geo& g, const DevSection& sd,
                 tan = mat.p[1];
                 sig = mat.p[10];
             } else {
-                const int B = sv.s2_blk, k = steel02_up(c, deps) ? 0 : 6;
+                const int B = sv.s2_blk, k = steel02_up(c, deps) ? 0 : 7;
                 S2Curve cv;
                 cv.epsr = sv.s2d[(k + 0) * B + i];
                 cv.sigr = sv.s2d[(k + 1) * B + i];
@@ -90,6 +90,7 @@ __device__ __forceinline__ void fiber_phase3(const Geo& g, const DevSection& sd,
                 cv.dsig = sv.s2d[(k + 3) * B + i];
                 cv.R = sv.s2d[(k + 4) * B + i];
                 cv.invR = sv.s2d[(k + 5) * B + i];
+                cv.rdenom = sv.s2d[(k + 6) * B + i];
                 steel02_curve_eval(mat, cv, eps, sig, tan);
             }
             double* o = fo + 2 * (ip * n_tot + j);
@@ -250,15 +251,21 @@ __device__ __forceinline__ bool sec_flex3(const double* r, double* f) {
 // ---- small dense algebra ------------------------------------------------------------------
 
 // _invert_5x5_flat_into: Gauss-Jordan with partial pivoting on a (destroyed); false when a
-// pivot column's largest magnitude is <= 1e-40.
+// pivot column's largest magnitude is <= 1e-40.  Everything unrolled, so the matrices stay in
+// registers (row exchanges by selects), and one reciprocal per pivot: of a pivot row's ten
+// divisions most had a zero numerator (413 cycles each), and the rolled form kept both matrices in
+// local memory.
 __device__ __forceinline__ bool invert5(double* a, double* inv) {
 #pragma unroll
     for (int i = 0; i < 25; ++i) inv[i] = 0.0;
 #pragma unroll
     for (int i = 0; i < 5; ++i) inv[i * 5 + i] = 1.0;
+    bool ok = true;
+#pragma unroll
     for (int i = 0; i < 5; ++i) {
         int pivot = i;
         double max_val = fabs(a[i * 5 + i]);
+#pragma unroll
         for (int r = i + 1; r < 5; ++r) {
             const double v = fabs(a[r * 5 + i]);
             if (v > max_val) {
@@ -266,33 +273,39 @@ __device__ __forceinline__ bool invert5(double* a, double* inv) {
                 pivot = r;
             }
         }
-        if (max_val <= 1.0e-40) return false;
+        if (max_val <= 1.0e-40) ok = false;
         if (pivot != i) {
-            for (int c = 0; c < 5; ++c) {
-                double t = a[i * 5 + c];
-                a[i * 5 + c] = a[pivot * 5 + c];
-                a[pivot * 5 + c] = t;
-                t = inv[i * 5 + c];
-                inv[i * 5 + c] = inv[pivot * 5 + c];
-                inv[pivot * 5 + c] = t;
+#pragma unroll
+            for (int r = i + 1; r < 5; ++r) {
+                const bool here = r == pivot;
+#pragma unroll
+                for (int c = 0; c < 5; ++c) {
+                    const double t = a[i * 5 + c], u = inv[i * 5 + c];
+                    a[i * 5 + c] = here ? a[r * 5 + c] : t;
+                    a[r * 5 + c] = here ? t : a[r * 5 + c];
+                    inv[i * 5 + c] = here ? inv[r * 5 + c] : u;
+                    inv[r * 5 + c] = here ? u : inv[r * 5 + c];
+                }
             }
         }
-        const double piv = a[i * 5 + i];
+        const double piv = a[i * 5 + i], rp = 1.0 / piv;
+#pragma unroll
         for (int c = 0; c < 5; ++c) {
-            a[i * 5 + c] /= piv;
-            inv[i * 5 + c] /= piv;
+            a[i * 5 + c] = quot(a[i * 5 + c], piv, rp);
+            inv[i * 5 + c] = quot(inv[i * 5 + c], piv, rp);
         }
+#pragma unroll
         for (int r = 0; r < 5; ++r) {
             if (r == i) continue;
             const double factor = a[r * 5 + i];
-            if (factor == 0.0) continue;
+#pragma unroll
             for (int c = 0; c < 5; ++c) {
                 a[r * 5 + c] -= factor * a[i * 5 + c];
                 inv[r * 5 + c] -= factor * inv[i * 5 + c];
             }
         }
     }
-    return true;
+    return ok;
 }
 
 // Local axes (rows x, y, z) from the end coordinates and vecxz (utils.mojo:59-140): default
@@ -631,7 +644,7 @@ __device__ void element3d_process(const Geo& g, const DevSection& sd, const DevE
     derive_element(g, sd, E, sv, fs.c2 + 4 * fs.c2_n + E.c2_off, const_cast<double*>(sv.c2d),
                    const_cast<double*>(sv.s2d));
     const int n_tot = sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el;
-    double* ys = const_cast<double*>(sv.s2d) + 12 * E.s2_blk;
+    double* ys = const_cast<double*>(sv.s2d) + 14 * E.s2_blk;
     double* zs = ys + ((n_tot + 1) & ~1);
     double* fo = zs + ((n_tot + 1) & ~1);
     for (int gg = tid; gg < n_tot; gg += blockDim.x) {

@@ -118,7 +118,7 @@ struct StageView {
     const double* s1;   // 5 fields x s1_blk
     const double* c1;   // 6 fields x c1_blk
     const double* c2d;  // C2Derived, 5 fields x c2_blk (shared-memory views only)
-    const double* s2d;  // S2Derived, 12 fields x s2_blk (shared-memory views only)
+    const double* s2d;  // S2Derived, 14 fields x s2_blk (shared-memory views only)
     int c2_blk, s2_blk, s1_blk, c1_blk;
 };
 
@@ -192,12 +192,13 @@ __device__ __forceinline__ void derive_s2(const Geo& g, const DevSection& sd, co
     S2Curve cv;
     steel02_curve_of(m, t, cv);
     const int B = sv.s2_blk;
-    s2d[(6 * k + 0) * B + idx] = cv.epsr;
-    s2d[(6 * k + 1) * B + idx] = cv.sigr;
-    s2d[(6 * k + 2) * B + idx] = cv.denom;
-    s2d[(6 * k + 3) * B + idx] = cv.dsig;
-    s2d[(6 * k + 4) * B + idx] = cv.R;
-    s2d[(6 * k + 5) * B + idx] = cv.invR;
+    s2d[(7 * k + 0) * B + idx] = cv.epsr;
+    s2d[(7 * k + 1) * B + idx] = cv.sigr;
+    s2d[(7 * k + 2) * B + idx] = cv.denom;
+    s2d[(7 * k + 3) * B + idx] = cv.dsig;
+    s2d[(7 * k + 4) * B + idx] = cv.R;
+    s2d[(7 * k + 5) * B + idx] = cv.invR;
+    s2d[(7 * k + 6) * B + idx] = cv.rdenom;
 }
 
 __device__ __forceinline__ void derive_element(const Geo& g, const DevSection& sd, const DevElem& E,
@@ -456,7 +457,7 @@ __device__ __forceinline__ void fiber_phase(const Geo& g, const DevSection& sd,
                 tan = mat.p[1];
                 sig = mat.p[10];
             } else {
-                const int B = sv.s2_blk, k = steel02_up(c, deps) ? 0 : 6;
+                const int B = sv.s2_blk, k = steel02_up(c, deps) ? 0 : 7;
                 S2Curve cv;
                 cv.epsr = sv.s2d[(k + 0) * B + idx];
                 cv.sigr = sv.s2d[(k + 1) * B + idx];
@@ -464,6 +465,7 @@ __device__ __forceinline__ void fiber_phase(const Geo& g, const DevSection& sd,
                 cv.dsig = sv.s2d[(k + 3) * B + idx];
                 cv.R = sv.s2d[(k + 4) * B + idx];
                 cv.invR = sv.s2d[(k + 5) * B + idx];
+                cv.rdenom = sv.s2d[(k + 6) * B + idx];
                 steel02_curve_eval(mat, cv, eps, sig, tan);
             }
             double* o = fo + 2 * (ip * n_tot + j);
@@ -1279,7 +1281,7 @@ __global__ void __launch_bounds__(kTeamThreads) element_state_kernel(
     StageView sv;
     stage_layout(E, smem_fib, sv);
     const int n_tot = sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el;
-    double* ys = const_cast<double*>(sv.s2d) + 12 * E.s2_blk;
+    double* ys = const_cast<double*>(sv.s2d) + 14 * E.s2_blk;
     double* fo = ys + ((n_tot + 1) & ~1);
     int err = ELEM_ERR_NONE;
     const uint32_t stage_bytes = stage_issue(E, fs, smem_fib, &bar, sv, fo);

@@ -12,7 +12,7 @@
 // between calls.  That is what lets the element kernels keep trial fiber state out of HBM.
 #pragma once
 
-#include <cstdint>
+#include "quotient.cuh"
 
 namespace strut {
 
@@ -33,6 +33,9 @@ enum {
     C2K_SIGMR = 2,  // Ec0 epsr
     C2K_EPS0T = 3,  // ft / Ec0
     C2K_EPSUT = 4,  // ft (1/Ets + 1/Ec0)
+    C2K_REPSC0 = 5, // 1 / epsc0
+    C2K_TSOFT = 6,  // (fcu - fc) / (epscu - epsc0)
+    C2K_RSOFT = 7,  // 1 / (epscu - epsc0)
     // Steel02
     S2K_ESH = 0,       // b E0
     S2K_EPSY = 1,      // Fy / E0
@@ -41,6 +44,7 @@ enum {
     S2K_DNEG = 4,      // 2 (a2 epsy)
     S2K_E0MESH = 5,    // E0 - Esh
     S2K_ESHEPSY = 6,   // Esh epsy
+    S2K_REPSY = 7,     // 1 / epsy
     // Steel01
     S1K_H = 0,         // (b E0) / (1 - b)
     S1K_EH = 1,        // (E0 H) / (E0 + H)
@@ -152,12 +156,12 @@ __device__ __forceinline__ void c2_compr_envlp(const DevMat& m, double strain, d
                                                double& tan) {
     const double fc = m.p[0], epsc0 = m.p[1], fcu = m.p[2], epscu = m.p[3];
     if (strain >= epsc0) {
-        double rat = strain / epsc0;
+        const double rat = quot(strain, epsc0, m.k[C2K_REPSC0]);
         sig = fc * rat * (2.0 - rat);
         tan = m.k[C2K_EC0] * (1.0 - rat);
     } else if (strain > epscu) {
-        sig = (fcu - fc) * (strain - epsc0) / (epscu - epsc0) + fc;
-        tan = (fcu - fc) / (epscu - epsc0);
+        sig = quot((fcu - fc) * (strain - epsc0), epscu - epsc0, m.k[C2K_RSOFT]) + fc;
+        tan = m.k[C2K_TSOFT];
     } else {
         sig = fcu;
         tan = 1.0e-10;
@@ -194,12 +198,12 @@ __device__ __forceinline__ void concrete02_derive(const DevMat& m, const C2State
     double tmm;
     c2_compr_envlp(m, c.ecmin, d.sigmm, tmm);
     d.er = (d.sigmm - m.k[C2K_SIGMR]) / (c.ecmin - m.k[C2K_EPSR]);
-    d.ept = c.ecmin - d.sigmm / d.er;
+    d.ept = c.ecmin - quot(d.sigmm, d.er, 1.0 / d.er);
     d.epn = d.ept + c.dept;
     double sicn, tcn;
     c2_tens_envlp(m, c.dept, sicn, tcn);
     d.etn = m.k[C2K_EC0];
-    if (c.dept != 0.0) d.etn = sicn / c.dept;
+    if (c.dept != 0.0) d.etn = quot(sicn, c.dept, 1.0 / c.dept);
 }
 
 // Stress and tangent for strain >= ecmin (unloading / reloading / tension branches).
@@ -276,6 +280,7 @@ __device__ __forceinline__ void concrete02_sig_tan(const DevMat& m, const C2Stat
 struct S2Curve {
     double epsr, sigr;
     double denom;  // epss0 - epsr
+    double rdenom; // 1 / denom
     double dsig;   // sigs0 - sigr
     double R, invR;
 };
@@ -342,11 +347,12 @@ __device__ __forceinline__ void steel02_branch(const DevMat& m, const S2State& c
 __device__ __forceinline__ void steel02_curve_of(const DevMat& m, const S2State& t, S2Curve& cv) {
     const double R0 = m.p[3], cR1 = m.p[4], cR2 = m.p[5];
     const double epsy = m.k[S2K_EPSY];
-    const double xi = fabs((t.epspl - t.epss0) / epsy);
-    const double R = R0 * (1.0 - (cR1 * xi) / (cR2 + xi));
+    const double xi = fabs(quot(t.epspl - t.epss0, epsy, m.k[S2K_REPSY]));
+    const double R = R0 * (1.0 - quot(cR1 * xi, cR2 + xi, 1.0 / (cR2 + xi)));
     cv.epsr = t.epsr;
     cv.sigr = t.sigr;
     cv.denom = t.epss0 - t.epsr;
+    cv.rdenom = 1.0 / cv.denom;
     cv.dsig = t.sigs0 - t.sigr;
     cv.R = R;
     cv.invR = 1.0 / R;
@@ -356,13 +362,16 @@ __device__ __forceinline__ void steel02_curve_of(const DevMat& m, const S2State&
 __device__ __forceinline__ void steel02_curve_eval(const DevMat& m, const S2Curve& cv, double eps,
                                                    double& sig, double& tan) {
     const double b = m.p[2];
-    const double epsrat = (eps - cv.epsr) / cv.denom;
+    const double epsrat = quot(eps - cv.epsr, cv.denom, cv.rdenom);
     const double dum1 = 1.0 + pow(fabs(epsrat), cv.R);
-    const double dum2 = pow(dum1, cv.invR);
-    double s = b * epsrat + (1.0 - b) * epsrat / dum2;
+    // far from the yield point |epsrat|^R vanishes beside 1, and 1^x is 1
+    const double dum2 = dum1 == 1.0 ? 1.0 : pow(dum1, cv.invR);
+    // dum2 overflows in a local iteration that diverges: the quotient is then 0, not quot's NaN
+    const double r2 = 1.0 / dum2, n2 = (1.0 - b) * epsrat;
+    double s = b * epsrat + (dum2 <= 1.7976931348623157e308 ? quot(n2, dum2, r2) : n2 * r2);
     s = s * cv.dsig + cv.sigr;
     double e = b + (1.0 - b) / (dum1 * dum2);
-    e = e * cv.dsig / cv.denom;
+    e = quot(e * cv.dsig, cv.denom, cv.rdenom);
     sig = s;
     tan = e;
 }

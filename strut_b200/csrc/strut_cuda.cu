@@ -70,6 +70,9 @@ DevMat make_devmat(const StrutUniMaterial& m) {
         d.k[C2K_SIGMR] = Ec0 * d.k[C2K_EPSR];
         d.k[C2K_EPS0T] = ft / Ec0;
         d.k[C2K_EPSUT] = ft * (1.0 / Ets + 1.0 / Ec0);
+        d.k[C2K_REPSC0] = 1.0 / epsc0;
+        d.k[C2K_TSOFT] = (fcu - fc) / (epscu - epsc0);
+        d.k[C2K_RSOFT] = 1.0 / (epscu - epsc0);
     } else if (m.type == STRUT_MAT_STEEL02) {
         const double Fy = p[0], E0 = p[1], b = p[2], a2 = p[7], a4 = p[9];
         const double Esh = b * E0, epsy = Fy / E0;
@@ -80,6 +83,7 @@ DevMat make_devmat(const StrutUniMaterial& m) {
         d.k[S2K_DNEG] = 2.0 * (a2 * epsy);
         d.k[S2K_E0MESH] = E0 - Esh;
         d.k[S2K_ESHEPSY] = Esh * epsy;
+        d.k[S2K_REPSY] = 1.0 / epsy;
     } else if (m.type == STRUT_MAT_CONCRETE01) {
         d.k[C1K_EC0] = (2.0 * p[0]) / p[1];
     } else if (m.type == STRUT_MAT_STEEL01) {
@@ -1039,12 +1043,12 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             c1_total += E.c1_blk;
             h->max_nip = std::max(h->max_nip, E.nip);
             // staged history (Concrete02 without dept) + derived constants (Concrete02 5, Steel02
-            // 12 doubles per fiber) + the section's fiber y + per-fiber stress and tangent of
+            // 14 doubles per fiber) + the section's fiber y + per-fiber stress and tangent of
             // every point
             const int n_tot = sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el;
             const size_t smem = 8 * (size_t)(4 * E.c2_blk + 10 * E.s2_blk + 5 * E.s1_blk + 6 * E.c1_blk) +
                                 4 * (size_t)E.s2_blk +
-                                8 * (size_t)(5 * E.c2_blk + 12 * E.s2_blk) +
+                                8 * (size_t)(5 * E.c2_blk + 14 * E.s2_blk) +
                                 8 * (size_t)((three_d ? 2 : 1) * ((n_tot + 1) & ~1) + 2 * E.nip * n_tot);
             h->elem_smem = std::max(h->elem_smem, smem);
             h->elem_fibers.push_back((long long)E.nip * (sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el));
