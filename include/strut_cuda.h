@@ -357,13 +357,13 @@ void* strut_gpu_stream(const StrutHandle* h);
  *                schemes x four subdivision levels, force_beam_column2d.mojo:1669-1763, each
  *                from the accepted state) on twelve CTAs at once, and the first success in
  *                Strut's order is kept; 0: the attempts run one after another.  Default 1.
- *   commit_team  threads per integration point in the commit kernel, 64 or 128 (default 128
- *                for up to 5 points, else 64; 128 needs at most 5 points).
+ *   commit_team  threads per integration point in the commit kernel, 64 (default) or 128
+ *                (at most 5 points).
  *   factor_ctas  CTAs of the cooperative wide-band factorisation (1 .. its resident limit;
  *                0: the default, as many as one panel has trailing tiles).
- *   element_threads  threads of an element CTA: 640 (default, one CTA per SM: the shortest
- *                per-element iteration), 320, 224 or 160 (2D only): as many CTAs per SM as
- *                registers and shared memory allow, more elements in flight.
+ *   element_threads  threads of an element CTA: 640 (one CTA per SM), 320 (default), 224 or 160
+ *                (2D only): as many CTAs per SM as registers and shared memory allow, more
+ *                elements in flight.
  * strut_gpu_set_tuning with t = NULL restores the defaults. */
 typedef struct StrutTuning {
     int32_t fan_out;

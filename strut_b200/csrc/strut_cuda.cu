@@ -401,8 +401,6 @@ static int prof_end(StrutHandle* h, int k) {
     return STRUT_OK;
 }
 
-// Element state kernel: kTeamThreads threads per element CTA.  Commit kernel: one team of 128
-// threads per integration point up to 5 points, else 64.
 using CommitKernel = decltype(&commit_kernel<128>);
 using ElemKernel = decltype(&element_state_kernel<2>);
 using InstKernel = decltype(&instance_newton_kernel<false>);
@@ -412,9 +410,13 @@ using InstKernel = decltype(&instance_newton_kernel<false>);
 static bool elem_threads_ok(const StrutHandle* h, int t) {
     return t == kTeamThreads || t == kTeamThreads / 2 || t == 224 || (t == 160 && h->ndf_all != 6);
 }
+// The default is 320: two elements share an SM and an element alone takes no longer.  Launches of
+// the element kernel with 640 / 320 / 224 threads (us): one 3x3 frame 35.5 / 34.4 / 35.0, 8 frames (447
+// elements) 71 / 53 / 55, 128 frames (7,204) 766 / 452 / 469, 32 4-story 3D frames (5,120) 1,217 / 703
+// / 750, a 12-story 3D frame (780) 220 / 152 / 156.
 static int elem_threads_of(const StrutHandle* h) {
     return h->tune.element_threads != 0 && elem_threads_ok(h, h->tune.element_threads) ? h->tune.element_threads
-                                                                                        : kTeamThreads;
+                                                                                        : kTeamThreads / 2;
 }
 static ElemKernel elem_kernel_of(const StrutHandle* h) {
     return h->ndf_all == 6 ? element_state_kernel<3> : element_state_kernel<2>;
@@ -436,7 +438,9 @@ static int elem_grid_of(StrutHandle* h) {
 static int commit_team_of(const StrutHandle* h) {
     // the commit kernel is launched with at most kTeamThreads threads: team x points
     if (h->tune.commit_team == 64 || (h->tune.commit_team == 128 && h->max_nip <= 5)) return h->tune.commit_team;
-    return h->max_nip <= 5 ? 128 : 64;
+    // 64 threads a point: more elements in flight.  128 / 64 (us): one 3x3 frame 15.7 / 15.7, 128 frames
+    // 361 / 211, 32 4-story 3D frames 328 / 225
+    return 64;
 }
 static CommitKernel commit_kernel_of(const StrutHandle* h) {
     return commit_team_of(h) == 128 ? commit_kernel<128> : commit_kernel<64>;
