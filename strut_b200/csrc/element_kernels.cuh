@@ -1809,62 +1809,82 @@ __global__ void __launch_bounds__(kTeamThreads) commit_kernel(
     __syncthreads();
     const int nip = E.nip;
     const bool three_d = E.nd == 12;
-    if (team < nip) {
-        // strain of a fiber: eps0 - y kappa (2D); eps0 + z kappa_y - y kappa_z (3D)
+    {
+        // Fibers of all points flattened over the CTA: the Steel02 fibers (two powers each) on warps
+        // of their own, the other families on the rest, so neither waits for the other; a thread's
+        // next fiber is loaded while it computes one, and fields that keep their bits are not
+        // written back.
         const double* es = estate + (size_t)e * kEStride;
-        const double eps0 = three_d ? es[kE3e + team] : es[kEe + team];
-        const double kappa = three_d ? es[kE3z + team] : es[kEk + team];
-        const double kappa_y = three_d ? es[kE3y + team] : 0.0;
-        const double* gz = three_d ? g.z : nullptr;
-        auto strain = [&](int gi) {
+        // strain of a fiber of point ip: eps0 - y kappa (2D); eps0 + z kappa_y - y kappa_z (3D)
+        auto strain = [&](int ip, int gi) {
             const double y = __ldg(g.y + gi);
-            return three_d ? eps0 + __ldg(gz + gi) * kappa_y - y * kappa : eps0 - y * kappa;
+            return three_d ? es[kE3e + ip] + __ldg(g.z + gi) * es[kE3y + ip] - y * es[kE3z + ip]
+                           : es[kEe + ip] - y * es[kEk + ip];
         };
-        int base = sd.geo_off;
-        for (int j = r; j < sd.n_s2; j += TEAM) {
-            const long long idx = E.s2_off + team * sd.n_s2 + j;
-            double* F = fs.s2 + idx;
+        const int w = tid >> 5, nw = blockDim.x >> 5, ws = steel_warps(nip * sd.n_s2, nw);
+        if (w < ws) {
             const long long N = fs.s2_n;
-            S2State c, t;
-            c.eps = F[0 * N]; c.sig = F[1 * N]; c.tan = F[2 * N]; c.epsmin = F[3 * N];
-            c.epsmax = F[4 * N]; c.epspl = F[5 * N]; c.epss0 = F[6 * N]; c.sigs0 = F[7 * N];
-            c.epsr = F[8 * N]; c.sigr = F[9 * N]; c.kon = fs.s2_kon[idx];
-            steel02_trial(g.mats[__ldg(g.m + base + j)], c, strain(base + j), t);
-            F[0 * N] = t.eps; F[1 * N] = t.sig; F[2 * N] = t.tan; F[3 * N] = t.epsmin;
-            F[4 * N] = t.epsmax; F[5 * N] = t.epspl; F[6 * N] = t.epss0; F[7 * N] = t.sigs0;
-            F[8 * N] = t.epsr; F[9 * N] = t.sigr; fs.s2_kon[idx] = t.kon;
-        }
-        base += sd.n_s2;
-        for (int j = r; j < sd.n_c2; j += TEAM) {
-            const long long idx = E.c2_off + team * sd.n_c2 + j;
-            double* F = fs.c2 + idx;
-            const long long N = fs.c2_n;
-            C2State c, t;
-            c.eps = F[0]; c.sig = F[N]; c.tan = F[2 * N]; c.ecmin = F[3 * N]; c.dept = F[4 * N];
-            concrete02_trial(g.mats[__ldg(g.m + base + j)], c, strain(base + j), t);
-            F[0] = t.eps; F[N] = t.sig; F[2 * N] = t.tan; F[3 * N] = t.ecmin; F[4 * N] = t.dept;
-        }
-        base += sd.n_c2;
-        for (int j = r; j < sd.n_s1; j += TEAM) {
-            const long long idx = E.s1_off + team * sd.n_s1 + j;
-            double* F = fs.s1 + idx;
-            const long long N = fs.s1_n;
-            S1State c, t;
-            c.eps = F[0]; c.sig = F[N]; c.tan = F[2 * N]; c.epsp = F[3 * N]; c.alpha = F[4 * N];
-            steel01_trial(g.mats[__ldg(g.m + base + j)], c, strain(base + j), t);
-            F[0] = t.eps; F[N] = t.sig; F[2 * N] = t.tan; F[3 * N] = t.epsp; F[4 * N] = t.alpha;
-        }
-        base += sd.n_s1;
-        for (int j = r; j < sd.n_c1; j += TEAM) {
-            const long long idx = E.c1_off + team * sd.n_c1 + j;
-            double* F = fs.c1 + idx;
-            const long long N = fs.c1_n;
-            C1State c, t;
-            c.eps = F[0]; c.sig = F[N]; c.tan = F[2 * N]; c.emin = F[3 * N]; c.eend = F[4 * N];
-            c.slope = F[5 * N];
-            concrete01_trial(g.mats[__ldg(g.m + base + j)], c, strain(base + j), t);
-            F[0] = t.eps; F[N] = t.sig; F[2 * N] = t.tan; F[3 * N] = t.emin; F[4 * N] = t.eend;
-            F[5 * N] = t.slope;
+            for (int i = tid; i < nip * sd.n_s2; i += 32 * ws) {
+                const int ip = i / sd.n_s2, j = i - ip * sd.n_s2;
+                double* F = fs.s2 + E.s2_off + i;
+                int* K = fs.s2_kon + E.s2_off + i;
+                S2State c, t;
+                c.eps = F[0 * N]; c.sig = F[1 * N]; c.tan = F[2 * N]; c.epsmin = F[3 * N];
+                c.epsmax = F[4 * N]; c.epspl = F[5 * N]; c.epss0 = F[6 * N]; c.sigs0 = F[7 * N];
+                c.epsr = F[8 * N]; c.sigr = F[9 * N]; c.kon = *K;
+                steel02_trial(g.mats[__ldg(g.m + sd.geo_off + j)], c, strain(ip, sd.geo_off + j), t);
+                F[0 * N] = t.eps; F[1 * N] = t.sig; F[2 * N] = t.tan;
+                if (changed(t.epsmin, c.epsmin)) F[3 * N] = t.epsmin;
+                if (changed(t.epsmax, c.epsmax)) F[4 * N] = t.epsmax;
+                if (t.kon != c.kon) {  // a new branch
+                    F[5 * N] = t.epspl; F[6 * N] = t.epss0; F[7 * N] = t.sigs0;
+                    F[8 * N] = t.epsr; F[9 * N] = t.sigr; *K = t.kon;
+                }
+            }
+        } else {
+            const int r = tid - 32 * ws, nt = blockDim.x - 32 * ws;
+            const int b2 = sd.geo_off + sd.n_s2, b1 = b2 + sd.n_c2, b0 = b1 + sd.n_s1;
+            {
+                const long long N = fs.c2_n;
+                const int n = nip * sd.n_c2;
+                auto load = [&](int i, C2State& c) {
+                    const double* F = fs.c2 + E.c2_off + i;
+                    c.eps = F[0]; c.sig = F[N]; c.tan = F[2 * N]; c.ecmin = F[3 * N]; c.dept = F[4 * N];
+                };
+                C2State c, next;
+                if (r < n) load(r, next);
+                for (int i = r; i < n; i += nt) {
+                    c = next;
+                    if (i + nt < n) load(i + nt, next);
+                    const int ip = i / sd.n_c2, j = i - ip * sd.n_c2;
+                    C2State t;
+                    concrete02_trial(g.mats[__ldg(g.m + b2 + j)], c, strain(ip, b2 + j), t);
+                    double* F = fs.c2 + E.c2_off + i;
+                    F[0] = t.eps; F[N] = t.sig; F[2 * N] = t.tan;
+                    if (changed(t.ecmin, c.ecmin)) F[3 * N] = t.ecmin;
+                    if (changed(t.dept, c.dept)) F[4 * N] = t.dept;
+                }
+            }
+            for (int i = r; i < nip * sd.n_s1; i += nt) {
+                const int ip = i / sd.n_s1, j = i - ip * sd.n_s1;
+                double* F = fs.s1 + E.s1_off + i;
+                const long long N = fs.s1_n;
+                S1State c, t;
+                c.eps = F[0]; c.sig = F[N]; c.tan = F[2 * N]; c.epsp = F[3 * N]; c.alpha = F[4 * N];
+                steel01_trial(g.mats[__ldg(g.m + b1 + j)], c, strain(ip, b1 + j), t);
+                F[0] = t.eps; F[N] = t.sig; F[2 * N] = t.tan; F[3 * N] = t.epsp; F[4 * N] = t.alpha;
+            }
+            for (int i = r; i < nip * sd.n_c1; i += nt) {
+                const int ip = i / sd.n_c1, j = i - ip * sd.n_c1;
+                double* F = fs.c1 + E.c1_off + i;
+                const long long N = fs.c1_n;
+                C1State c, t;
+                c.eps = F[0]; c.sig = F[N]; c.tan = F[2 * N]; c.emin = F[3 * N]; c.eend = F[4 * N];
+                c.slope = F[5 * N];
+                concrete01_trial(g.mats[__ldg(g.m + b0 + j)], c, strain(ip, b0 + j), t);
+                F[0] = t.eps; F[N] = t.sig; F[2 * N] = t.tan; F[3 * N] = t.emin; F[4 * N] = t.eend;
+                F[5 * N] = t.slope;
+            }
         }
     }
     if (three_d) {
@@ -1908,7 +1928,7 @@ __global__ void __launch_bounds__(kTeamThreads) commit_kernel(
     if (E.type != 3 || E.rec < 0 || !rec_out) return;
     __syncthreads();
     // dispBeamColumn2d recorder: section evaluation at the converged displacements from the
-    // just-committed state (each thread reads back exactly the fibers it wrote)
+    // just-committed state (written above by this CTA, before the barrier)
     const double L = E.L, inv_L = 1.0 / L, inv_L_sq = inv_L * inv_L;
     if (team < nip) {
         const double xi = E.xi[team];

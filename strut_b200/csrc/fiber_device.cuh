@@ -197,13 +197,13 @@ struct C2Derived {
 __device__ __forceinline__ void concrete02_derive(const DevMat& m, const C2State& c, C2Derived& d) {
     double tmm;
     c2_compr_envlp(m, c.ecmin, d.sigmm, tmm);
-    d.er = (d.sigmm - m.k[C2K_SIGMR]) / (c.ecmin - m.k[C2K_EPSR]);
-    d.ept = c.ecmin - quot(d.sigmm, d.er, 1.0 / d.er);
+    d.er = quot(d.sigmm - m.k[C2K_SIGMR], c.ecmin - m.k[C2K_EPSR]);
+    d.ept = c.ecmin - quot(d.sigmm, d.er);
     d.epn = d.ept + c.dept;
     double sicn, tcn;
     c2_tens_envlp(m, c.dept, sicn, tcn);
     d.etn = m.k[C2K_EC0];
-    if (c.dept != 0.0) d.etn = quot(sicn, c.dept, 1.0 / c.dept);
+    if (c.dept != 0.0) d.etn = quot(sicn, c.dept);
 }
 
 // Stress and tangent for strain >= ecmin (unloading / reloading / tension branches).
@@ -348,14 +348,14 @@ __device__ __forceinline__ void steel02_curve_of(const DevMat& m, const S2State&
     const double R0 = m.p[3], cR1 = m.p[4], cR2 = m.p[5];
     const double epsy = m.k[S2K_EPSY];
     const double xi = fabs(quot(t.epspl - t.epss0, epsy, m.k[S2K_REPSY]));
-    const double R = R0 * (1.0 - quot(cR1 * xi, cR2 + xi, 1.0 / (cR2 + xi)));
+    const double R = R0 * (1.0 - quot(cR1 * xi, cR2 + xi));
     cv.epsr = t.epsr;
     cv.sigr = t.sigr;
     cv.denom = t.epss0 - t.epsr;
-    cv.rdenom = 1.0 / cv.denom;
+    cv.rdenom = recip(cv.denom);
     cv.dsig = t.sigs0 - t.sigr;
     cv.R = R;
-    cv.invR = 1.0 / R;
+    cv.invR = quot(1.0, R);
 }
 
 // Menegotto-Pinto curve: stress and tangent at eps on the branch cv.
@@ -367,8 +367,8 @@ __device__ __forceinline__ void steel02_curve_eval(const DevMat& m, const S2Curv
     // far from the yield point |epsrat|^R vanishes beside 1, and 1^x is 1
     const double dum2 = dum1 == 1.0 ? 1.0 : pow(dum1, cv.invR);
     // dum2 overflows in a local iteration that diverges: the quotient is then 0, not quot's NaN
-    const double r2 = 1.0 / dum2, n2 = (1.0 - b) * epsrat;
-    double s = b * epsrat + (dum2 <= 1.7976931348623157e308 ? quot(n2, dum2, r2) : n2 * r2);
+    const double n2 = (1.0 - b) * epsrat;
+    double s = b * epsrat + (dum2 <= 1.7976931348623157e308 ? quot(n2, dum2) : n2 / dum2);
     s = s * cv.dsig + cv.sigr;
     double e = b + (1.0 - b) / (dum1 * dum2);
     e = quot(e * cv.dsig, cv.denom, cv.rdenom);
@@ -461,6 +461,12 @@ __device__ __forceinline__ void steel01_trial(const DevMat& m, const S1State& c,
     t.alpha = c.alpha + H * dg * sgn;
     t.sig = sigma_trial - E0 * dg * sgn;
     t.tan = m.k[S1K_EH];
+}
+
+// Whether a state field has to be written: its bits changed (most of a history does not from one
+// state to the next: Concrete02's ecmin and dept, Steel02's branch).
+__device__ __forceinline__ bool changed(double a, double b) {
+    return __double_as_longlong(a) != __double_as_longlong(b);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -13,9 +13,8 @@
 // instances, a multiple of the tile), so every field of a tile of kFsTile consecutive instances
 // is one contiguous, 16-byte aligned run: one bulk copy per field and tile.
 //
-// Warp-specialised CTAs, several per SM: kFsTile instance warps share the tile's Concrete02,
-// Steel01, Concrete01 and elastic fibers (flattened over the tile's instances, so the warps' last
-// round is nearly full), and W_s steel warps take the Steel02 fibers of all the tile's instances
+// Warp-specialised CTAs, several per SM: kFsTile instance warps take the Concrete02, Steel01,
+// Concrete01 and elastic fibers of one instance of the tile each, and W_s steel warps take the Steel02 fibers of all the tile's instances
 // together, so the expensive Menegotto-Pinto branch runs on full warps instead of a few lanes of
 // every warp.  Two stages: the TMA unit (cp.async.bulk, mbarrier completion, no multicast) brings
 // tile k + 2 into a stage as soon as every warp has read tile k from it.  The warps hand work to
@@ -48,8 +47,7 @@ struct FsLayout {
     int stage_doubles;                            // one stage, kon included, a multiple of 2
     int steel_warps;                              // W_s (0 without Steel02 fibers)
     int n_mats;                                   // materials of the batch
-    int n_oth;                                    // non-Steel02 fibers of a section
-    float inv_s2, inv_oth;                        // 1 / n_s2, 1 / n_oth
+    float inv_s2;                                 // 1 / n_s2
     uint32_t bytes_s2, bytes_c2, bytes_s1, bytes_c1, bytes_kon, bytes_total;  // per field / tile
 };
 
@@ -75,9 +73,7 @@ __host__ __device__ inline FsLayout fs_layout(const DevSection& sd) {
     const int ws = (T * sd.n_s2 + 31) / 32;
     L.steel_warps = ws < kFsMaxSteelWarps ? ws : kFsMaxSteelWarps;
     L.n_mats = 0;
-    L.n_oth = L.n_tot - sd.n_s2;
     L.inv_s2 = sd.n_s2 ? 1.0f / sd.n_s2 : 0.0f;
-    L.inv_oth = L.n_oth ? 1.0f / L.n_oth : 0.0f;
     L.bytes_s2 = 8u * T * L.p_s2;
     L.bytes_c2 = 8u * T * L.p_c2;
     L.bytes_s1 = 8u * T * L.p_s1;
@@ -164,7 +160,9 @@ __device__ __forceinline__ void fs_other_fiber(const FsGeo& G, const BatchState&
         concrete02_trial(mat, c, e, t);
         if (commit) {
             double* Gp = bs.c2 + i * L.p_c2 + jj;
-            Gp[0] = t.eps; Gp[N3] = t.sig; Gp[2 * N3] = t.tan; Gp[3 * N3] = t.ecmin; Gp[4 * N3] = t.dept;
+            Gp[0] = t.eps; Gp[N3] = t.sig; Gp[2 * N3] = t.tan;
+            if (changed(t.ecmin, c.ecmin)) Gp[3 * N3] = t.ecmin;
+            if (changed(t.dept, c.dept)) Gp[4 * N3] = t.dept;
         }
         sA = t.sig * A;
         tA = t.tan * A;
@@ -326,7 +324,6 @@ __global__ void __launch_bounds__(32 * (kFsTile + kFsMaxSteelWarps), 2)
     if (warp < T) {
         // ---- instance warps: the tile's non-Steel02 fibers, then (one warp per tile) the sums
         const int w = warp;
-        const int n_items = T * L.n_oth;
         double ek_cur = strains(t0);
         for (int k = 0;; ++k) {
             const long long t = t0 + k * G_;
@@ -343,17 +340,17 @@ __global__ void __launch_bounds__(32 * (kFsTile + kFsMaxSteelWarps), 2)
             if (ok && k >= 2) ok = __all_sync(all, mbar_wait_bounded(&bar_summed[s], par ^ 1u));
             if (!ok) break;
             if (threadIdx.x == 0) pend &= ~(1u << s);
-            for (int base = w * 32; base < n_items; base += 32 * T) {
-                const int q = base + lane;
-                const int inst = q < n_items ? fs_div(q, L.n_oth, L.inv_oth) : 0;
-                const double e0 = __shfl_sync(all, ek_here, 2 * inst), ka = __shfl_sync(all, ek_here, 2 * inst + 1);
-                if (q >= n_items || inst >= n_valid) continue;
-                const int j = L.n_s2 + (q - inst * L.n_oth);
-                double sA, tA;
-                fs_other_fiber(G, bs, L, st, inst, t * T + inst, j, e0, ka, N3, N1, N4, commit, sA, tA);
-                double* f = fk + (size_t)inst * 2 * L.n_tot;
-                f[2 * j] = sA;
-                f[2 * j + 1] = tA;
+            // warp w takes instance w: a section's fibers over 32 lanes need as many rounds as the
+            // tile's over all lanes, with one strain pair and without index arithmetic
+            const double e0 = __shfl_sync(all, ek_here, 2 * w), ka = __shfl_sync(all, ek_here, 2 * w + 1);
+            if (w < n_valid) {
+                double* f = fk + (size_t)w * 2 * L.n_tot;
+                for (int j = L.n_s2 + lane; j < L.n_tot; j += 32) {
+                    double sA, tA;
+                    fs_other_fiber(G, bs, L, st, w, t * T + w, j, e0, ka, N3, N1, N4, commit, sA, tA);
+                    f[2 * j] = sA;
+                    f[2 * j + 1] = tA;
+                }
             }
             __syncwarp();
             if (lane == 0) {
@@ -420,10 +417,14 @@ __global__ void __launch_bounds__(32 * (kFsTile + kFsMaxSteelWarps), 2)
                 steel02_trial(G.mats[G.m[j]], c, e0 - y * ka, tr);
                 if (commit) {
                     double* Gp = bs.s2 + i * L.p_s2 + j;
-                    Gp[0] = tr.eps; Gp[N2] = tr.sig; Gp[2 * N2] = tr.tan; Gp[3 * N2] = tr.epsmin;
-                    Gp[4 * N2] = tr.epsmax; Gp[5 * N2] = tr.epspl; Gp[6 * N2] = tr.epss0; Gp[7 * N2] = tr.sigs0;
-                    Gp[8 * N2] = tr.epsr; Gp[9 * N2] = tr.sigr;
-                    bs.kon[i * L.p_s2 + j] = tr.kon;
+                    Gp[0] = tr.eps; Gp[N2] = tr.sig; Gp[2 * N2] = tr.tan;
+                    if (changed(tr.epsmin, c.epsmin)) Gp[3 * N2] = tr.epsmin;
+                    if (changed(tr.epsmax, c.epsmax)) Gp[4 * N2] = tr.epsmax;
+                    if (tr.kon != c.kon) {  // a new branch
+                        Gp[5 * N2] = tr.epspl; Gp[6 * N2] = tr.epss0; Gp[7 * N2] = tr.sigs0;
+                        Gp[8 * N2] = tr.epsr; Gp[9 * N2] = tr.sigr;
+                        bs.kon[i * L.p_s2 + j] = tr.kon;
+                    }
                 }
                 double* f = fk + (size_t)inst * 2 * L.n_tot;
                 f[2 * j] = tr.sig * A;
