@@ -81,7 +81,7 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
 #pragma unroll 1
     for (; k + bw < n; ++k) {
         const double akk = *pk, rkk = rk[k & 1], pa_ = fabs(akk);
-        if (flag[2 * ((k + 1) & 1)]) return verdict(k - 1);  // raised in step k - 1
+        const int failed = flag[2 * ((k + 1) & 1)];  // raised in step k - 1
         double f[NR], uk[NC], a[NR][NC];
 #pragma unroll
         for (int u = 0; u < NR; ++u) f[u] = *pf[u];
@@ -91,6 +91,7 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
 #pragma unroll
             for (int u = 0; u < NR; ++u) a[u][v] = *pa[u][v];
         }
+        if (failed) return verdict(k - 1);
         bool swap = false;
 #pragma unroll
         for (int u = 0; u < NR; ++u) {

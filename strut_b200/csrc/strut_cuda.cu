@@ -9,8 +9,7 @@
 //     instance_newton_kernel    assembly gather, residual, band factor/solve, update, test
 //     (host reads the number of still-active instances)
 //   commit_kernel               fiber commit, basic-deformation sync, element-force records
-//   post_step_kernel            Newmark velocity / acceleration update
-//   record_disp_kernel          displacement records
+//   post_step_kernel            Newmark velocity / acceleration update, displacement records
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -326,6 +325,8 @@ struct StrutHandle {
     InstArrays A;
     int* d_free_inst = nullptr;
     int* d_free_dir = nullptr;
+    int* d_elem_inst = nullptr;  // instance of each element
+    int* d_iter_done = nullptr;  // IterCheck::done
     int* d_rec_dof = nullptr;
     int* d_rece_base = nullptr;
     int* d_elem_err = nullptr;
@@ -560,7 +561,7 @@ static int launch_instances(StrutHandle* h, int mode, int step) {
     A.bytes_counter = h->d_counters + 4;
     TRY(prof_begin(h));
     TRY(launch_gather(h, h->d_insts, mode));
-    inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, mode, step);
+    inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, mode, IterCheck{nullptr, nullptr, 0});
     CK(cudaGetLastError());
     TRY(launch_large(h, mode, nullptr, &A));
     TRY(prof_end(h, 1));
@@ -647,8 +648,8 @@ static int add_while_node(cudaGraphNode_t* node, cudaGraph_t g, const cudaGraphN
 
 // The whole step loop as one CUDA graph: an outer WHILE over steps (condition set by
 // step_end_kernel) around predictor -> inner WHILE over Newton iterations (element state
-// determination, instance Newton kernel, newton_check_kernel sets the condition) -> commit ->
-// Newmark update -> displacement records -> step_end.  The host synchronises once per run.
+// determination, instance Newton kernel, whose last CTA sets the condition) -> commit, beside it
+// Newmark update and displacement records -> step_end.  The host synchronises once per run.
 static int build_graph(StrutHandle* h) {
     if (h->gexec) {
         cudaGraphExecDestroy(h->gexec);
@@ -669,15 +670,15 @@ static int build_graph(StrutHandle* h) {
     CK(cudaGraphConditionalHandleCreate(&inner, body, 1, cudaGraphCondAssignDefault));
     const int nF = h->n_free_total;
     const int tb = 256;
-    const int npred = std::max(nF, h->n_inst);
+    const int npred = std::max(std::max(nF, h->n_inst), h->n_elem);
     InstArrays A = h->A;
     A.hist_iters = h->d_hist_iters;
     A.ctl = h->d_ctl;
     A.bytes_counter = h->d_counters + 4;
-    cudaGraphNode_t n_pred, n_inner, n_commit, n_post, n_rec, n_end;
+    cudaGraphNode_t n_pred, n_inner, n_commit, n_post, n_end;
     TRY(add_kernel_node(&n_pred, body, nullptr, 0, predictor_kernel, dim3((npred + tb - 1) / tb), dim3(tb), 0,
                         (const DevInst*)h->d_insts, A, (const int*)h->d_free_inst, (const int*)h->d_free_dir,
-                        (const double*)h->d_ag, nF, h->n_inst, h->d_ctl, inner, 1));
+                        (const int*)h->d_elem_inst, h->n_elem, (const double*)h->d_ag, nF, h->n_inst, h->d_ctl, inner, 1));
     cudaGraph_t ibody;
     cudaGraphNode_t n_before_inner = n_pred;
     if (h->any_chain || h->pred) {
@@ -696,7 +697,7 @@ static int build_graph(StrutHandle* h) {
     }
     if (h->pred) TRY(pred_add_nodes(h, body, n_before_inner, &n_before_inner));
     TRY(add_while_node(&n_inner, body, &n_before_inner, 1, inner, &ibody));
-    cudaGraphNode_t n_el, n_in, n_chk;
+    cudaGraphNode_t n_el, n_in;
     TRY(add_kernel_node(&n_el, ibody, nullptr, 0, elem_kernel_of(h), dim3(h->elem_grid),
                         elem_block(h), h->elem_smem, (const DevElem*)h->d_elems, h->geo,
                         h->fs, (const double*)h->A.u_full, h->d_estate, h->d_ek, h->d_ef,
@@ -717,10 +718,8 @@ static int build_graph(StrutHandle* h) {
         n_after_el = n_g;
     }
     TRY(add_kernel_node(&n_in, ibody, &n_after_el, 1, inst_kernel_of(h), dim3(h->n_inst), dim3(256),
-                        h->inst_smem, (const DevInst*)h->d_insts, A, (int)INST_MODE_NEWTON, 0));
-    cudaGraphNode_t n_before_chk = n_in;
-    TRY(add_kernel_node(&n_chk, ibody, &n_before_chk, 1, newton_check_kernel, dim3(1), dim3(32), 0, h->d_ctl,
-                        (const int*)h->A.nactive, inner, 1));
+                        h->inst_smem, (const DevInst*)h->d_insts, A, (int)INST_MODE_NEWTON,
+                        IterCheck{h->d_iter_done, h->d_ctl, inner}));
     TRY(add_kernel_node(&n_commit, body, &n_inner, 1, commit_kernel_of(h), dim3(h->n_elem),
                         commit_block(h), 0, (const DevElem*)h->d_elems, h->geo, h->fs,
                         (const double*)h->A.u_full, h->d_estate, (const int*)h->A.status, h->d_hist_ef,
@@ -735,15 +734,11 @@ static int build_graph(StrutHandle* h) {
                             (int)ELEM_MODE_RECORD, h->n_elem, rec_pass_of(h)));
         n_after_commit = n_rp;
     }
-    TRY(add_kernel_node(&n_post, body, &n_after_commit, 1, post_step_kernel, dim3((nF + tb - 1) / tb), dim3(tb), 0,
-                        (const DevInst*)h->d_insts, A, (const int*)h->d_free_inst, nF));
-    cudaGraphNode_t last = n_post;
-    if (h->n_rec_total > 0) {
-        TRY(add_kernel_node(&n_rec, body, &n_post, 1, record_disp_kernel, dim3((h->n_rec_total + tb - 1) / tb),
-                            dim3(tb), 0, (const double*)h->A.u_full, (const int*)h->d_rec_dof, h->n_rec_total,
-                            h->d_hist_disp, (const DevCtl*)h->d_ctl));
-        last = n_rec;
-    }
+    const int npost = std::max(nF, h->n_rec_total);
+    TRY(add_kernel_node(&n_post, body, &n_inner, 1, post_step_kernel, dim3((npost + tb - 1) / tb), dim3(tb), 0,
+                        (const DevInst*)h->d_insts, A, (const int*)h->d_free_inst, nF, (const int*)h->d_rec_dof,
+                        h->n_rec_total, h->d_hist_disp, (const DevCtl*)h->d_ctl));
+    cudaGraphNode_t last = n_after_commit;
     if (h->n_sec_slots > 0) {
         cudaGraphNode_t n_sec;
         TRY(add_kernel_node(&n_sec, body, &last, 1, record_sections_kernel, dim3((h->n_sec_slots * 32 + 255) / 256),
@@ -752,7 +747,8 @@ static int build_graph(StrutHandle* h) {
                             h->ndf_all == 6 ? 4 : 2, h->d_hist_sec, (const DevCtl*)h->d_ctl));
         last = n_sec;
     }
-    TRY(add_kernel_node(&n_end, body, &last, 1, step_end_kernel, dim3(1), dim3(256), 0, h->d_ctl,
+    const cudaGraphNode_t before_end[2] = {last, n_post};
+    TRY(add_kernel_node(&n_end, body, before_end, 2, step_end_kernel, dim3(1), dim3(256), 0, h->d_ctl,
                         (const int*)h->A.status, h->d_fail_step, h->n_inst, h->A.nactive, h->A.el, outer, 1));
     CK(cudaGraphInstantiate(&h->gexec, g, 0));
     h->graph_keys[0] = h->d_hist_disp;
@@ -1524,6 +1520,11 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         A.sl_coef = d_slc;
         h->n_slaves_total = (int)sl_dof.size();
     }
+    {
+        std::vector<int> ei(elems.size());
+        for (size_t e = 0; e < elems.size(); ++e) ei[e] = elems[e].inst;
+        if ((rc = upload(&h->d_elem_inst, ei, al)) || (rc = dzeros(&h->d_iter_done, 1, al))) return bail(rc);
+    }
     if ((rc = dzeros(&h->d_ctl, 1, al))) return bail(rc);
     {
         std::vector<int> neg(h->n_inst, -1);
@@ -1621,7 +1622,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         InstArrays B = A;
         B.export_band = d_Kinit;
         if ((rc = launch_gather(h, d_tmp, INST_MODE_EXPORT)) != STRUT_OK) return bail(rc);
-        inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(d_tmp, B, INST_MODE_EXPORT, -1);
+        inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(d_tmp, B, INST_MODE_EXPORT, IterCheck{nullptr, nullptr, 0});
         CK(cudaGetLastError());
         if ((rc = launch_large(h, INST_MODE_EXPORT, d_tmp, &B)) != STRUT_OK) return bail(rc);
         if (any_kinit) {
@@ -1721,10 +1722,11 @@ int strut_gpu_run_steps(StrutHandle* h, int32_t n_steps, StrutStepStats* stats) 
         cudaGraphConditionalHandle none = 0;
         for (int s = 0; s < n_steps; ++s) {
             const int step = step0 + s;
-            const int npred = std::max(nF, h->n_inst);
+            const int npred = std::max(std::max(nF, h->n_inst), h->n_elem);
             TRY(prof_begin(h));
             predictor_kernel<<<(npred + tb - 1) / tb, tb, 0, h->stream>>>(
-                h->d_insts, h->A, h->d_free_inst, h->d_free_dir, h->d_ag, nF, h->n_inst, h->d_ctl, none, 0);
+                h->d_insts, h->A, h->d_free_inst, h->d_free_dir, h->d_elem_inst, h->n_elem, h->d_ag, nF, h->n_inst,
+                h->d_ctl, none, 0);
             CK(cudaGetLastError());
             if (h->any_chain || h->pred) {
                 copy_doubles_kernel<<<592, tb, 0, h->stream>>>(h->d_estate, h->A.estate_base,
@@ -1744,7 +1746,7 @@ int strut_gpu_run_steps(StrutHandle* h, int32_t n_steps, StrutStepStats* stats) 
             for (int it = 0; it < h->max_iters_global; ++it) {
                 TRY(launch_elements(h));
                 TRY(launch_instances(h, INST_MODE_NEWTON, step));
-                newton_check_kernel<<<1, 32, 0, h->stream>>>(h->d_ctl, h->A.nactive, none, 0);
+                newton_check_kernel<<<1, 32, 0, h->stream>>>(h->d_ctl);
                 CK(cudaGetLastError());
                 int n_act = 0;
                 CK(cudaMemcpyAsync(&n_act, h->A.nactive, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -1759,15 +1761,12 @@ int strut_gpu_run_steps(StrutHandle* h, int32_t n_steps, StrutStepStats* stats) 
             TRY(launch_record_pass(h));
             TRY(prof_end(h, 2));
             TRY(prof_begin(h));
-            post_step_kernel<<<(nF + tb - 1) / tb, tb, 0, h->stream>>>(h->d_insts, h->A, h->d_free_inst, nF);
+            const int npost = std::max(nF, h->n_rec_total);
+            post_step_kernel<<<(npost + tb - 1) / tb, tb, 0, h->stream>>>(
+                h->d_insts, h->A, h->d_free_inst, nF, h->d_rec_dof, h->n_rec_total, h->d_hist_disp, h->d_ctl);
             CK(cudaGetLastError());
             TRY(prof_end(h, 4));
             if (h->prof) h->P.bytes[2] += h->commit_bytes_total;
-            if (h->n_rec_total > 0) {
-                record_disp_kernel<<<(h->n_rec_total + tb - 1) / tb, tb, 0, h->stream>>>(
-                    h->A.u_full, h->d_rec_dof, h->n_rec_total, h->d_hist_disp, h->d_ctl);
-                CK(cudaGetLastError());
-            }
             if (h->n_sec_slots > 0) {
                 record_sections_kernel<<<(h->n_sec_slots * 32 + 255) / 256, 256, 0, h->stream>>>(
                     h->d_elems, h->geo, h->fs, h->A.u_full, h->d_estate, h->d_secrec, h->n_sec_slots,
@@ -2069,7 +2068,7 @@ int strut_gpu_factor_solve(StrutHandle* h, const double* rhs, double* du) {
     A.rhs_in = h->d_rhs;
     std::vector<int> zeros(h->n_inst, 0);
     CK(cudaMemcpyAsync(h->A.status, zeros.data(), sizeof(int) * h->n_inst, cudaMemcpyHostToDevice, h->stream));
-    inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, INST_MODE_SOLVE_EXPORTED, -1);
+    inst_kernel_of(h)<<<h->n_inst, 256, h->inst_smem, h->stream>>>(h->d_insts, A, INST_MODE_SOLVE_EXPORTED, IterCheck{nullptr, nullptr, 0});
     CK(cudaGetLastError());
     TRY(launch_large(h, INST_MODE_SOLVE_EXPORTED, nullptr, &A));
     CK(cudaStreamSynchronize(h->stream));
