@@ -6,7 +6,7 @@
 //
 // A 2D frame's system (36 to 216 unknowns, half band 11 to 20) is a chain of n dependent steps of a
 // few hundred operations, so the time is the latency of a step.  Measured for 216 unknowns of half
-// band 20 (cycles per unknown): factorisation 1,230 -> 355, back substitution 810 -> 263 (the sums of a row
+// band 20 (cycles per unknown): factorisation 1,230 -> 261, back substitution 810 -> 263 (the sums of a row
 // taken column by column instead, 123, rounded differently and were dropped: a batch of long records
 // is chaotic at the rounding level, and one record of 256 ended elsewhere).
 #pragma once
@@ -20,6 +20,7 @@ constexpr int kBackWarpMax = 24;   // widest half band of the one-warp back subs
 constexpr int kBackWarpGroup = 8;  // unknowns per window position
 constexpr int kLuRowsMax = 62;     // widest half band of band_lu_cta
 constexpr int kLuRowsThreads = 256;
+constexpr int kNoColumn = 0x7fffffff;  // no column of the factorisation failed
 
 // Barrier of the first nt threads of the CTA (a multiple of 32).
 __device__ __forceinline__ void bar_first(int nt) { asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory"); }
@@ -32,29 +33,26 @@ __device__ __forceinline__ void bar_first(int nt) { asm volatile("bar.sync 1, %0
 // entry receives the reference's operations in the reference's order.  KEEP: multipliers stored.
 //
 // What bounds it is the chain of a step (load, quotient, multiply-add, reciprocal, barrier), and
-// next to it the instructions of a warp that works alone on its scheduler.  So the step has no
-// inner loop, no division (74 cycles, 413 with a zero numerator, which bands are full of; recip 40,
-// quot 24) and no reducing barrier (63 against 28 cycles): a row that needs an interchange raises a
-// flag that the next step reads with its other operands.  Flags alternate between two places by the
-// step's parity: a place is written in one step and read in the next only, so all warps leave the
-// loop at the same step.  While all bw rows exist, every operand
-// has a pointer that moves by a fixed stride; rows and columns that a warp or lane does not have
-// point at the zeros z (stride 0) instead of being tested.
-// NR NW >= bw, 32 NC > bw.  rk: 2 doubles; z: 2 doubles; flag: 4 ints of shared memory.  Returns
-// 0 ok, 2 singular, 6 a row swap would be needed (the caller then starts again from the assembled
-// values), on the threads of the first NW warps.
+// next to it the instructions of a warp that works alone on its scheduler.  So a step is straight
+// code without a branch: no inner loop, no division (74 cycles, 413 with a zero numerator, which
+// bands are full of; recip 40, quot 24), no reducing barrier (63 against 28 cycles), and the pivot
+// test only folds the first failing column into a key that is looked at after the last step (as
+// flags that end the loop it cost 120 of 375 cycles a step).  Every operand has a pointer that moves
+// by a fixed stride; rows and columns that a warp or lane does not have point at the zeros z (stride
+// 0), and bw rows of zeros behind the band (B has n + bw rows) stand in for the rows the last steps
+// lack.
+// NR NW >= bw, 32 NC > bw.  rk: 2 doubles; z: 2 doubles; key: an int, all of shared memory; the first
+// failing column comes back in *key.
 template <int NR, int NC, int NW, bool KEEP>
-__device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, int woff, double* rk, double* z,
-                                            int* flag) {
-    constexpr int NT = 32 * NW;
+__device__ __forceinline__ void band_lu_rows(double* B, int n, int bw, int rw, int woff, double* rk, double* z,
+                                            int* key) {
+    constexpr int NT = 32 * NW, kNone = kNoColumn;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         rk[0] = recip(B[bw]);
         z[0] = z[1] = 0.0;
-        flag[0] = flag[1] = flag[2] = flag[3] = 0;
+        *key = kNone;
     }
-    // what step k of an elimination that cannot go on means: a row swap (6) or a singular matrix
-    auto verdict = [&](int k) { return flag[2 * (k & 1)] && flag[2 * (k & 1) + 1] ? 6 : 2; };
     const double* pf[NR];  // B(i, k) of this warp's rows
     double* pa[NR][NC];    // this lane's entries of them
     const double* pu[NC];  // and of row k
@@ -76,12 +74,11 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
             sa[u][v] = r > bw ? 0 : su[v];
         }
     }
+    int first = kNone;  // 2 k: column k needs a swap; 2 k + 1: column k is singular
     bar_first(NT);
-    int k = 0;
 #pragma unroll 1
-    for (; k + bw < n; ++k) {
-        const double akk = *pk, rkk = rk[k & 1], pa_ = fabs(akk);
-        const int failed = flag[2 * ((k + 1) & 1)];  // raised in step k - 1
+    for (int k = 0; k < n; ++k) {
+        const double akk = *pk, rkk = rk[k & 1], d = fabs(akk), dbig = fmax(d, 1.0e-14);
         double f[NR], uk[NC], a[NR][NC];
 #pragma unroll
         for (int u = 0; u < NR; ++u) f[u] = *pf[u];
@@ -91,11 +88,11 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
 #pragma unroll
             for (int u = 0; u < NR; ++u) a[u][v] = *pa[u][v];
         }
-        if (failed) return verdict(k - 1);
-        bool swap = false;
+        // pivot search of linear_solver_backend.mojo:640-657: an entry strictly larger than the
+        // diagonal selects another row, and the largest one decides singularity (1e-14)
+        bool swap = d <= 1.0e-14, big = false;
 #pragma unroll
         for (int u = 0; u < NR; ++u) {
-            swap = swap || fabs(f[u]) > pa_;
             const double q = quot(f[u], akk, rkk);
 #pragma unroll
             for (int v = 0; v < NC; ++v) {
@@ -103,80 +100,49 @@ __device__ __forceinline__ int band_lu_rows(double* B, int n, int bw, int rw, in
                 *pa[u][v] = a[u][v];
                 pa[u][v] += sa[u][v];
             }
+            swap = swap || fabs(f[u]) > d;
+            big = big || fabs(f[u]) > dbig;
             if (KEEP && lane == 0 && sf[u]) *const_cast<double*>(pf[u]) = q;
             pf[u] += sf[u];
         }
-        if (threadIdx.x == 0) rk[(k + 1) & 1] = recip(a[0][0]);
-        if (swap) {
-            // pivot search of linear_solver_backend.mojo:640-657: an entry strictly larger than
-            // the diagonal selects another row; the largest one decides singularity
-            flag[2 * (k & 1)] = 1;
-#pragma unroll
-            for (int u = 0; u < NR; ++u)
-                if (fabs(f[u]) > 1.0e-14) flag[2 * (k & 1) + 1] = 1;
-        }
+        const double rn = recip(a[0][0]);
+        if (threadIdx.x == 0) rk[(k + 1) & 1] = rn;
+        first = min(first, big ? 2 * k : swap ? 2 * k + 1 : kNone);
 #pragma unroll
         for (int v = 0; v < NC; ++v) pu[v] += su[v];
         pk += rw;
         bar_first(NT);
-        if (pa_ <= 1.0e-14) return verdict(k);
     }
-    if (k > 0 && flag[2 * ((k + 1) & 1)]) return verdict(k - 1);
-    // the last bw columns, fewer rows and columns each
-    int dk = k * rw + bw;
-#pragma unroll 1
-    for (; k < n; ++k) {
-        const int m = n - 1 - k;
-        const double akk = B[dk], rkk = rk[k & 1], pa_ = fabs(akk);
-        double f[NR], uk[NC];
-        bool swap = false;
-#pragma unroll
-        for (int v = 0; v < NC; ++v) {
-            const int c = lane + 1 + 32 * v;
-            uk[v] = c <= m + 1 ? B[c <= m ? dk + c : woff + k] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < NR; ++u) {
-            const int r = 1 + warp + NW * u;
-            if (r > m) continue;
-            const int d = dk + r * (rw - 1);
-            f[u] = B[d];
-            swap = swap || fabs(f[u]) > pa_;
-            const double q = quot(f[u], akk, rkk);
-#pragma unroll
-            for (int v = 0; v < NC; ++v) {
-                const int c = lane + 1 + 32 * v;
-                if (c <= m + 1) {
-                    double* p = B + (c <= m ? d + c : woff + k + r);
-                    const double t = *p - q * uk[v];
-                    *p = t;
-                    if (u == 0 && v == 0 && threadIdx.x == 0) rk[(k + 1) & 1] = recip(t);
-                }
-            }
-            if (KEEP && lane == 0) B[d] = q;
-        }
-        if (swap) {
-            flag[2 * (k & 1)] = 1;
-#pragma unroll
-            for (int u = 0; u < NR; ++u)
-                if (1 + warp + NW * u <= m && fabs(f[u]) > 1.0e-14) flag[2 * (k & 1) + 1] = 1;
-        }
-        dk += rw;
-        bar_first(NT);
-        if (flag[2 * (k & 1)] || pa_ <= 1.0e-14) return verdict(k);
-    }
-    return 0;
+    first = __reduce_min_sync(0xffffffffu, first);
+    if (lane == 0) atomicMin(key, first);
+}
+
+// Rows of zeros that band_lu_rows needs behind the band; the limit on the shared memory of band and
+// vectors decides whether they fit (else band_lu_smem runs).
+constexpr size_t kBandSmemMax = 220 * 1024;
+__host__ __device__ inline int band_pad_rows(int n, int bw, int vectors) {
+    return bw <= kLuRowsMax &&
+                   ((size_t)(n + bw) * (2 * bw + 1) + (size_t)vectors * n) * sizeof(double) <= kBandSmemMax
+               ? bw : 0;
 }
 
 // band_lu_rows for half bands up to kLuRowsMax, by a CTA of kLuRowsThreads threads (all of them
-// call; the result is the same on all).
+// call).  Returns 0 ok, 2 singular, 6 a row swap would be needed (the caller then starts again from
+// the assembled values), the same on all threads.  Four warps up to half band 31 (measured at 14 / 20: 226 / 273
+// cycles a step against 253 / 286 with eight), eight above.
 template <bool KEEP>
 __device__ __forceinline__ int band_lu_cta(double* B, int n, int bw, int rw, int woff, double* rk, double* z,
-                                           int* flag) {
-    constexpr int NW = kLuRowsThreads / 32;
-    if (bw <= 2 * NW) return band_lu_rows<2, 1, NW, KEEP>(B, n, bw, rw, woff, rk, z, flag);
-    if (bw <= 3 * NW) return band_lu_rows<3, 1, NW, KEEP>(B, n, bw, rw, woff, rk, z, flag);
-    return band_lu_rows<8, 2, NW, KEEP>(B, n, bw, rw, woff, rk, z, flag);
+                                           int* key) {
+    if (bw > 31) {
+        band_lu_rows<8, 2, kLuRowsThreads / 32, KEEP>(B, n, bw, rw, woff, rk, z, key);
+    } else if (threadIdx.x < 128) {
+        if (bw <= 12) band_lu_rows<3, 1, 4, KEEP>(B, n, bw, rw, woff, rk, z, key);
+        else if (bw <= 16) band_lu_rows<4, 1, 4, KEEP>(B, n, bw, rw, woff, rk, z, key);
+        else if (bw <= 20) band_lu_rows<5, 1, 4, KEEP>(B, n, bw, rw, woff, rk, z, key);
+        else band_lu_rows<8, 1, 4, KEEP>(B, n, bw, rw, woff, rk, z, key);
+    }
+    __syncthreads();
+    return *key == kNoColumn ? 0 : *key & 1 ? 2 : 6;
 }
 
 // U x = w with one warp for bw <= kBackWarpMax, every row's sum in the reference's order (columns

@@ -13,7 +13,7 @@
 namespace strut {
 
 constexpr int kNoAllocMaxN = 512;               // largest system order accepted
-constexpr size_t kNoAllocSmemMax = 220 * 1024;  // band + 4 vectors in shared memory
+constexpr size_t kNoAllocSmemMax = kBandSmemMax;  // band + 4 vectors in shared memory
 
 // Shared by every call on a device and kept between calls.  Nothing in them has to start at
 // zero: a call writes every entry of the n x n work matrix and the n pivots before reading them.
@@ -35,11 +35,12 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
     __shared__ double red[32];
     __shared__ int red_r[32];
     __shared__ double s_rk[2], s_z[2];  // band_lu_cta
-    __shared__ int s_flag[4];
+    __shared__ int s_key;
     const int tid = threadIdx.x, nt = blockDim.x;
     const int rw = 2 * bw + 1;
     double* Kb = smem_one;
-    double* R = Kb + (size_t)n * rw;
+    const int pad = spd ? 0 : band_pad_rows(n, bw, 4);  // rows of zeros behind the band
+    double* R = Kb + (size_t)(n + pad) * rw;
     double* w = R + n;
     double* xs = w + n;
     double* fac = xs + n;
@@ -64,10 +65,11 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
     int rc;
     if (spd) {
         rc = band_chol_smem(Kb, n, bw, rw, fac);
-    } else if (bw <= kLuRowsMax) {
+    } else if (bw <= pad) {
         for (int i = tid; i < n; i += nt) w[i] = R[i];
+        for (int t = tid; t < pad * rw; t += nt) Kb[n * rw + t] = 0.0;
         __syncthreads();
-        rc = band_lu_cta<false>(Kb, n, bw, rw, (int)(w - Kb), s_rk, s_z, s_flag);
+        rc = band_lu_cta<false>(Kb, n, bw, rw, (int)(w - Kb), s_rk, s_z, &s_key);
         forward = true;
     } else {
         rc = band_lu_smem(Kb, n, bw, rw, fac);
@@ -131,7 +133,8 @@ extern "C" int strut_gpu_band_solve_noalloc(const double* band_dev, int32_t n, i
     if (half_bw < 0 || half_bw > n - 1) return fail(STRUT_BAD_ARG, "half_bw must be in 0..n-1");
     if (!band_dev || !rhs_dev || !x_dev || !status_dev) return fail(STRUT_BAD_ARG, "null pointer");
     const int rw = 2 * half_bw + 1;
-    const size_t smem = ((size_t)n * rw + 4 * (size_t)n) * sizeof(double);
+    const int pad = system == STRUT_SYSTEM_BAND_SPD ? 0 : strut::band_pad_rows(n, half_bw, 4);
+    const size_t smem = ((size_t)(n + pad) * rw + 4 * (size_t)n) * sizeof(double);
     int dev = 0;
     CK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kNoAllocMaxDevices) return fail(STRUT_UNSUPPORTED, "device index too large");

@@ -584,7 +584,7 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
     __shared__ int red_r[32];
     __shared__ int s_it;  // this instance's Newton iterations of the step so far
     __shared__ double s_rk[2], s_z[2];  // band_lu_cta
-    __shared__ int s_flag[4];
+    __shared__ int s_key;
     __shared__ __align__(16) double s_pbuf[PIVOT ? kPivotBuf : 2];
     const int inst = blockIdx.x;
     const int tid = threadIdx.x, nt = blockDim.x;
@@ -599,8 +599,9 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
     if (mode == INST_MODE_NEWTON && !A.active[inst]) return;
     int* hrow = (A.hist_iters && A.ctl) ? A.hist_iters + (size_t)A.ctl->step * gridDim.x : nullptr;
     const int n = I.n, bw = I.bw, rw = I.rw;
-    double* Kb = smem_inst;        // n * rw
-    double* vt = Kb + (size_t)n * rw;
+    double* Kb = smem_inst;        // n * rw, then the rows of zeros of band_lu_rows
+    const int pad = band_pad_rows(n, bw, 6);
+    double* vt = Kb + (size_t)(n + pad) * rw;
     double* R = vt + n;
     double* w = R + n;
     double* du = w + n;
@@ -855,12 +856,13 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
         __syncthreads();
     } else if (I.spd) {
         rc = band_chol_smem(Kb, n, bw, rw, fac);
-    } else if (bw <= kLuRowsMax) {
+    } else if (bw <= pad) {
         for (int i = tid; i < n; i += nt) w[i] = R[i];
+        for (int t = tid; t < pad * rw; t += nt) Kb[n * rw + t] = 0.0;
         __syncthreads();
         const int woff = (int)(w - Kb);
-        rc = modified ? band_lu_cta<true>(Kb, n, bw, rw, woff, s_rk, s_z, s_flag)
-                      : band_lu_cta<false>(Kb, n, bw, rw, woff, s_rk, s_z, s_flag);
+        rc = modified ? band_lu_cta<true>(Kb, n, bw, rw, woff, s_rk, s_z, &s_key)
+                      : band_lu_cta<false>(Kb, n, bw, rw, woff, s_rk, s_z, &s_key);
         forward = true;
     } else {
         rc = band_lu_smem(Kb, n, bw, rw, fac);

@@ -1324,7 +1324,8 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             h->max_large_bw = std::max(h->max_large_bw, bw);
             h->lfactor_smem = std::max(h->lfactor_smem, fsm);
         } else {
-            h->inst_smem = std::max(h->inst_smem, ismem);
+            const size_t pad = (size_t)band_pad_rows(nf, bw, 6);
+            h->inst_smem = std::max(h->inst_smem, ismem + pad * rw * sizeof(double));
         }
         h->insts[inst] = I;
         // excitations

@@ -1,4 +1,5 @@
-"""The band factor-solve in shared memory at the edges of its variants (half bands 8, 16, 24, 62),
+"""The band factor-solve in shared memory at the edges of its variants (half bands 12, 16, 20, 31,
+62, and bands that leave no room for the rows of zeros behind them),
 through strut_gpu_band_solve_noalloc, against a dense solve in numpy.
 
 The systems are diagonally dominant (condition number below 10), so a backward-stable elimination
@@ -41,6 +42,7 @@ def _solve(band, n, bw, system, rhs):
 
 @pytest.mark.parametrize("n,bw", [(1, 0), (2, 1), (7, 3), (8, 7), (9, 8), (31, 11), (32, 12), (33, 13), (40, 16),
                                   (65, 17), (216, 20), (100, 21), (64, 24), (257, 24), (500, 24), (64, 25),
+                                  (50, 31), (50, 32), (512, 25), (500, 25),
                                   (120, 40), (100, 61), (100, 62), (100, 63)])
 @pytest.mark.parametrize("spd", [False, True])
 def test_band_solve(n, bw, spd):
