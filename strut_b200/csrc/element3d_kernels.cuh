@@ -82,15 +82,8 @@ __device__ __forceinline__ void fiber_phase3(const Geo& g, const DevSection& sd,
                 tan = mat.p[1];
                 sig = mat.p[10];
             } else {
-                const int B = sv.s2_blk, k = steel02_up(c, deps) ? 0 : 7;
                 S2Curve cv;
-                cv.epsr = sv.s2d[(k + 0) * B + i];
-                cv.sigr = sv.s2d[(k + 1) * B + i];
-                cv.denom = sv.s2d[(k + 2) * B + i];
-                cv.dsig = sv.s2d[(k + 3) * B + i];
-                cv.R = sv.s2d[(k + 4) * B + i];
-                cv.invR = sv.s2d[(k + 5) * B + i];
-                cv.rdenom = sv.s2d[(k + 6) * B + i];
+                load_curve(sv, i, steel02_up(c, deps), cv);
                 steel02_curve_eval(mat, cv, eps, sig, tan);
             }
             double* o = fo + 2 * (ip * n_tot + j);
@@ -641,10 +634,8 @@ __device__ void element3d_process(const Geo& g, const DevSection& sd, const DevE
         }
         return;
     }
-    derive_element(g, sd, E, sv, fs.c2 + 4 * fs.c2_n + E.c2_off, const_cast<double*>(sv.c2d),
-                   const_cast<double*>(sv.s2d));
     const int n_tot = sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el;
-    double* ys = const_cast<double*>(sv.s2d) + 14 * E.s2_blk;
+    double* ys = sv.tail;
     double* zs = ys + ((n_tot + 1) & ~1);
     double* fo = zs + ((n_tot + 1) & ~1);
     for (int gg = tid; gg < n_tot; gg += blockDim.x) {

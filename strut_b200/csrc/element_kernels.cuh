@@ -2,8 +2,8 @@
 //
 // One CTA per element (a persistent grid claiming elements from a list).  The element's
 // committed fiber history (all of its sections, all families) is staged into shared memory with
-// cp.async.bulk (the TMA unit's bulk copy) completing on an mbarrier, and the constants each
-// fiber's trial rule derives from its committed state are computed once per launch.  Every
+// cp.async.bulk (the TMA unit's bulk copy) completing on an mbarrier, together with the constants
+// each fiber's trial rule derives from its committed state (written by the commit).  Every
 // section evaluation of the element-level flexibility iteration then reads shared memory only,
 // in two phases: the trial stress and tangent of every fiber of every integration point (one
 // fiber per thread, Steel02 fibers on one warp per SM sub-partition), then the section sums in a
@@ -111,14 +111,14 @@ struct ElemScratch {
 // Family views of the element's committed history (shared memory, or global memory with the
 // family length as field stride).
 struct StageView {
-    const double* c2;   // staged: 4 fields x c2_blk (eps sig tan ecmin; dept only enters the
-                        // derived constants, which read it from a separate buffer)
-    const double* s2;   // 10 fields x s2_blk
+    const double* c2;   // 4 fields x c2_blk (eps sig tan ecmin); in a global view 5, with dept
+    const double* s2;   // staged: eps only; in a global view 10 fields x s2_blk
     const int* kon;     // s2_blk
     const double* s1;   // 5 fields x s1_blk
     const double* c1;   // 6 fields x c1_blk
     const double* c2d;  // C2Derived, 5 fields x c2_blk (shared-memory views only)
-    const double* s2d;  // S2Derived, 14 fields x s2_blk (shared-memory views only)
+    const double* s2d;  // the two S2Curves, 2 x 7 fields x s2_blk (shared-memory views only)
+    double* tail;       // shared memory behind the staged arrays
     int c2_blk, s2_blk, s1_blk, c1_blk;
 };
 
@@ -143,82 +143,52 @@ __device__ __forceinline__ void load_c2(const StageView& sv, int idx, C2State& c
     c.dept = 0.0;
 }
 
+// The staged Steel02 fields: strain and branch (the rest of the history is in the derived curves).
 __device__ __forceinline__ void load_s2(const StageView& sv, int idx, S2State& c) {
-    const int B = sv.s2_blk;
-    c.eps = sv.s2[0 * B + idx];
-    c.sig = sv.s2[1 * B + idx];
-    c.tan = sv.s2[2 * B + idx];
-    c.epsmin = sv.s2[3 * B + idx];
-    c.epsmax = sv.s2[4 * B + idx];
-    c.epspl = sv.s2[5 * B + idx];
-    c.epss0 = sv.s2[6 * B + idx];
-    c.sigs0 = sv.s2[7 * B + idx];
-    c.epsr = sv.s2[8 * B + idx];
-    c.sigr = sv.s2[9 * B + idx];
+    c.eps = sv.s2[idx];
     c.kon = sv.kon[idx];
 }
 
-// Derived constants of every Concrete02 / Steel02 fiber of the staged element, computed once
-// per launch by the whole CTA (the committed state does not change inside a launch).  A
-// Concrete02 fiber's dept comes from c2_dept: the element's dept field, in global memory or
-// copied into shared memory beside the staged history.  The two
-// branch curves of a Steel02 fiber (each with its own pow) are two work items, given to the last
-// threads of the CTA, so they run beside the Concrete02 items instead of after them.
-__device__ __forceinline__ void derive_c2(const Geo& g, const DevSection& sd, const StageView& sv,
-                                          const double* __restrict__ c2_dept, double* c2d, int idx) {
-    C2State c;
-    load_c2(sv, idx, c);
-    c.dept = c2_dept[idx];
-    const int j = idx % sd.n_c2;
-    C2Derived d;
-    concrete02_derive(g.mats[__ldg(g.m + sd.geo_off + sd.n_s2 + j)], c, d);
-    const int B = sv.c2_blk;
-    c2d[0 * B + idx] = d.sigmm;
-    c2d[1 * B + idx] = d.er;
-    c2d[2 * B + idx] = d.ept;
-    c2d[3 * B + idx] = d.epn;
-    c2d[4 * B + idx] = d.etn;
+__device__ __forceinline__ void load_curve(const StageView& sv, int idx, bool up, S2Curve& cv) {
+    const double* p = sv.s2d + (up ? 0 : 7) * sv.s2_blk + idx;
+    const int B = sv.s2_blk;
+    cv.epsr = p[0];
+    cv.sigr = p[B];
+    cv.denom = p[2 * B];
+    cv.dsig = p[3 * B];
+    cv.R = p[4 * B];
+    cv.invR = p[5 * B];
+    cv.rdenom = p[6 * B];
 }
 
-// Branch curve k (0: strain increasing, 1: decreasing) of Steel02 fiber idx (steel02_derive).
-__device__ __forceinline__ void derive_s2(const Geo& g, const DevSection& sd, const StageView& sv, double* s2d,
-                                          int idx, int k) {
-    S2State c;
-    load_s2(sv, idx, c);
-    const int j = idx % sd.n_s2;
-    const DevMat& m = g.mats[__ldg(g.m + sd.geo_off + j)];
+// The constants a fiber's trial rule derives from its committed state change only when that state
+// does, so the commit (and the initial state) writes them beside the history and the element kernel
+// stages them: deriving them at every state determination took 6.5 K of its 39 K cycles.  Element
+// block layout (FiberState::c2d, s2d): fields of a block behind one another, one bulk copy each.
+__device__ __forceinline__ void store_c2d(const DevMat& m, const C2State& c, double* D, int B) {
+    C2Derived d;
+    concrete02_derive(m, c, d);
+    D[0] = d.sigmm;
+    D[B] = d.er;
+    D[2 * B] = d.ept;
+    D[3 * B] = d.epn;
+    D[4 * B] = d.etn;
+}
+
+// Branch curve of a Steel02 fiber whose strain increases (up) or decreases next.
+__device__ __forceinline__ void store_s2d(const DevMat& m, const S2State& c, bool up, double* D, int B) {
     S2State t;
-    steel02_branch(m, c, k == 0, t);
+    steel02_branch(m, c, up, t);
     S2Curve cv;
     steel02_curve_of(m, t, cv);
-    const int B = sv.s2_blk;
-    s2d[(7 * k + 0) * B + idx] = cv.epsr;
-    s2d[(7 * k + 1) * B + idx] = cv.sigr;
-    s2d[(7 * k + 2) * B + idx] = cv.denom;
-    s2d[(7 * k + 3) * B + idx] = cv.dsig;
-    s2d[(7 * k + 4) * B + idx] = cv.R;
-    s2d[(7 * k + 5) * B + idx] = cv.invR;
-    s2d[(7 * k + 6) * B + idx] = cv.rdenom;
-}
-
-__device__ __forceinline__ void derive_element(const Geo& g, const DevSection& sd, const DevElem& E,
-                                               const StageView& sv, const double* __restrict__ c2_dept,
-                                               double* c2d, double* s2d) {
-    const int nc = E.nip * sd.n_c2, ns2 = 2 * E.nip * sd.n_s2;
-    const int nt = blockDim.x, tid = threadIdx.x;
-    if (ns2 > 0 && ns2 <= nt / 2) {
-        // Concrete02 on the first nt - ns2 threads, one Steel02 branch on each of the others
-        const int split = nt - ns2;
-        if (tid < split) {
-            for (int idx = tid; idx < nc; idx += split) derive_c2(g, sd, sv, c2_dept, c2d, idx);
-        } else {
-            const int q = tid - split;
-            derive_s2(g, sd, sv, s2d, q >> 1, q & 1);
-        }
-        return;
-    }
-    for (int idx = tid; idx < nc; idx += nt) derive_c2(g, sd, sv, c2_dept, c2d, idx);
-    for (int q = tid; q < ns2; q += nt) derive_s2(g, sd, sv, s2d, q >> 1, q & 1);
+    double* p = D + (up ? 0 : 7) * B;
+    p[0] = cv.epsr;
+    p[B] = cv.sigr;
+    p[2 * B] = cv.denom;
+    p[3 * B] = cv.dsig;
+    p[4 * B] = cv.R;
+    p[5 * B] = cv.invR;
+    p[6 * B] = cv.rdenom;
 }
 
 __device__ __forceinline__ void acc_fiber(double* a, double fs, double ks, double y) {
@@ -457,15 +427,8 @@ __device__ __forceinline__ void fiber_phase(const Geo& g, const DevSection& sd,
                 tan = mat.p[1];
                 sig = mat.p[10];
             } else {
-                const int B = sv.s2_blk, k = steel02_up(c, deps) ? 0 : 7;
                 S2Curve cv;
-                cv.epsr = sv.s2d[(k + 0) * B + idx];
-                cv.sigr = sv.s2d[(k + 1) * B + idx];
-                cv.denom = sv.s2d[(k + 2) * B + idx];
-                cv.dsig = sv.s2d[(k + 3) * B + idx];
-                cv.R = sv.s2d[(k + 4) * B + idx];
-                cv.invR = sv.s2d[(k + 5) * B + idx];
-                cv.rdenom = sv.s2d[(k + 6) * B + idx];
+                load_curve(sv, idx, steel02_up(c, deps), cv);
                 steel02_curve_eval(mat, cv, eps, sig, tan);
             }
             double* o = fo + 2 * (ip * n_tot + j);
@@ -1033,8 +996,10 @@ __device__ __forceinline__ void copy_struct(T* dst, const T* src) {
 // wait.
 __device__ __forceinline__ void stage_layout(const DevElem& E, double* sm, StageView& sv) {
     double* c2 = sm;
-    double* s2 = c2 + 4 * E.c2_blk;
-    double* s1 = s2 + 10 * E.s2_blk;
+    double* c2d = c2 + 4 * E.c2_blk;
+    double* s2 = c2d + 5 * E.c2_blk;
+    double* s2d = s2 + E.s2_blk;
+    double* s1 = s2d + 14 * E.s2_blk;
     double* c1 = s1 + 5 * E.s1_blk;
     int* kon = reinterpret_cast<int*>(c1 + 6 * E.c1_blk);
     sv.c2 = c2;
@@ -1042,43 +1007,39 @@ __device__ __forceinline__ void stage_layout(const DevElem& E, double* sm, Stage
     sv.s1 = s1;
     sv.c1 = c1;
     sv.kon = kon;
-    // derived constants follow the staged history (kon occupies s2_blk ints, s2_blk % 4 == 0)
-    sv.c2d = reinterpret_cast<const double*>(kon + E.s2_blk);
-    sv.s2d = sv.c2d + 5 * E.c2_blk;
+    sv.c2d = c2d;
+    sv.s2d = s2d;
+    sv.tail = reinterpret_cast<double*>(kon + E.s2_blk);  // s2_blk % 4 == 0
     sv.c2_blk = E.c2_blk;
     sv.s2_blk = E.s2_blk;
     sv.s1_blk = E.s1_blk;
     sv.c1_blk = E.c1_blk;
 }
 
-// dept (optional): shared-memory destination of the Concrete02 dept field (E.c2_blk doubles,
-// 16-byte aligned), copied with the history.
 __device__ __forceinline__ uint32_t stage_issue(const DevElem& E, const FiberState& fs, double* sm,
-                                                uint64_t* bar, StageView& sv, double* dept = nullptr) {
+                                                uint64_t* bar, StageView& sv) {
     stage_layout(E, sm, sv);
-    double* c2 = const_cast<double*>(sv.c2);
-    double* s2 = const_cast<double*>(sv.s2);
-    double* s1 = const_cast<double*>(sv.s1);
-    double* c1 = const_cast<double*>(sv.c1);
-    int* kon = const_cast<int*>(sv.kon);
-    if (!E.c2_blk) dept = nullptr;
-    const uint32_t bytes = (uint32_t)(8 * (4 * E.c2_blk + 10 * E.s2_blk + 5 * E.s1_blk + 6 * E.c1_blk) +
-                                      4 * E.s2_blk + (dept ? 8 * E.c2_blk : 0));
+    const uint32_t bytes = (uint32_t)(8 * (9 * E.c2_blk + 15 * E.s2_blk + 5 * E.s1_blk + 6 * E.c1_blk) +
+                                      4 * E.s2_blk);
     if (bytes == 0) return 0u;
     if (threadIdx.x == 0) {
         // the previous element's reads of this buffer (generic proxy) come before the copies
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_arrive_expect_tx(bar, bytes);
-        for (int f = 0; f < 4 && E.c2_blk; ++f)
-            bulk_g2s(c2 + f * E.c2_blk, fs.c2 + f * fs.c2_n + E.c2_off, 8u * E.c2_blk, bar);
-        if (dept) bulk_g2s(dept, fs.c2 + 4 * fs.c2_n + E.c2_off, 8u * E.c2_blk, bar);
-        for (int f = 0; f < 10 && E.s2_blk; ++f)
-            bulk_g2s(s2 + f * E.s2_blk, fs.s2 + f * fs.s2_n + E.s2_off, 8u * E.s2_blk, bar);
-        if (E.s2_blk) bulk_g2s(kon, fs.s2_kon + E.s2_off, 4u * E.s2_blk, bar);
+        if (E.c2_blk) {
+            double* c2 = const_cast<double*>(sv.c2);
+            for (int f = 0; f < 4; ++f) bulk_g2s(c2 + f * E.c2_blk, fs.c2 + f * fs.c2_n + E.c2_off, 8u * E.c2_blk, bar);
+            bulk_g2s(const_cast<double*>(sv.c2d), fs.c2d + 5ll * E.c2_off, 40u * E.c2_blk, bar);
+        }
+        if (E.s2_blk) {
+            bulk_g2s(const_cast<double*>(sv.s2), fs.s2 + E.s2_off, 8u * E.s2_blk, bar);
+            bulk_g2s(const_cast<double*>(sv.s2d), fs.s2d + 14ll * E.s2_off, 112u * E.s2_blk, bar);
+            bulk_g2s(const_cast<int*>(sv.kon), fs.s2_kon + E.s2_off, 4u * E.s2_blk, bar);
+        }
         for (int f = 0; f < 5 && E.s1_blk; ++f)
-            bulk_g2s(s1 + f * E.s1_blk, fs.s1 + f * fs.s1_n + E.s1_off, 8u * E.s1_blk, bar);
+            bulk_g2s(const_cast<double*>(sv.s1) + f * E.s1_blk, fs.s1 + f * fs.s1_n + E.s1_off, 8u * E.s1_blk, bar);
         for (int f = 0; f < 6 && E.c1_blk; ++f)
-            bulk_g2s(c1 + f * E.c1_blk, fs.c1 + f * fs.c1_n + E.c1_off, 8u * E.c1_blk, bar);
+            bulk_g2s(const_cast<double*>(sv.c1) + f * E.c1_blk, fs.c1 + f * fs.c1_n + E.c1_off, 8u * E.c1_blk, bar);
     }
     return bytes;
 }
@@ -1275,16 +1236,15 @@ __global__ void __launch_bounds__(kTeamThreads) element_state_kernel(
         return;
     }
     __syncthreads();
-    // the bulk copies of the fiber history go out first, with the Concrete02 dept field into the
-    // buffer of the per-fiber results (free until the first evaluation); the element state and
-    // the section's fiber y are read while they are in flight
+    // the bulk copies of the fiber history go out first; the element state and the section's fiber y
+    // are read while they are in flight
     StageView sv;
     stage_layout(E, smem_fib, sv);
     const int n_tot = sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el;
-    double* ys = const_cast<double*>(sv.s2d) + 14 * E.s2_blk;
+    double* ys = sv.tail;
     double* fo = ys + ((n_tot + 1) & ~1);
     int err = ELEM_ERR_NONE;
-    const uint32_t stage_bytes = stage_issue(E, fs, smem_fib, &bar, sv, fo);
+    const uint32_t stage_bytes = stage_issue(E, fs, smem_fib, &bar, sv);
     {
         const double* es = estate + (size_t)e * kEStride;
         if (tid < E.nip) {
@@ -1351,8 +1311,6 @@ __global__ void __launch_bounds__(kTeamThreads) element_state_kernel(
         stop = true;
         return;
     }
-    derive_element(g, sd, E, sv, fo, const_cast<double*>(sv.c2d), const_cast<double*>(sv.s2d));
-    __syncthreads();
     const int nip = E.nip;
     if (E.type == 3) {
         // ---------------- dispBeamColumn2d ----------------
@@ -1836,10 +1794,15 @@ __global__ void __launch_bounds__(kTeamThreads) commit_kernel(
                 F[0 * N] = t.eps; F[1 * N] = t.sig; F[2 * N] = t.tan;
                 if (changed(t.epsmin, c.epsmin)) F[3 * N] = t.epsmin;
                 if (changed(t.epsmax, c.epsmax)) F[4 * N] = t.epsmax;
+                // the curve of a reversal starts from this state; the one of going on is the branch's
+                double* D = fs.s2d + 14ll * E.s2_off + i;
+                const DevMat& mat = g.mats[__ldg(g.m + sd.geo_off + j)];
                 if (t.kon != c.kon) {  // a new branch
                     F[5 * N] = t.epspl; F[6 * N] = t.epss0; F[7 * N] = t.sigs0;
                     F[8 * N] = t.epsr; F[9 * N] = t.sigr; *K = t.kon;
+                    store_s2d(mat, t, t.kon != 2, D, E.s2_blk);
                 }
+                if (t.kon == 1 || t.kon == 2 || t.kon != c.kon) store_s2d(mat, t, t.kon == 2, D, E.s2_blk);
             }
         } else {
             const int r = tid - 32 * ws, nt = blockDim.x - 32 * ws;
@@ -1861,8 +1824,11 @@ __global__ void __launch_bounds__(kTeamThreads) commit_kernel(
                     concrete02_trial(g.mats[__ldg(g.m + b2 + j)], c, strain(ip, b2 + j), t);
                     double* F = fs.c2 + E.c2_off + i;
                     F[0] = t.eps; F[N] = t.sig; F[2 * N] = t.tan;
-                    if (changed(t.ecmin, c.ecmin)) F[3 * N] = t.ecmin;
-                    if (changed(t.dept, c.dept)) F[4 * N] = t.dept;
+                    const bool ce = changed(t.ecmin, c.ecmin), cd = changed(t.dept, c.dept);
+                    if (ce) F[3 * N] = t.ecmin;
+                    if (cd) F[4 * N] = t.dept;
+                    if (ce || cd)
+                        store_c2d(g.mats[__ldg(g.m + b2 + j)], t, fs.c2d + 5ll * E.c2_off + i, E.c2_blk);
                 }
             }
             for (int i = r; i < nip * sd.n_s1; i += nt) {

@@ -4,8 +4,8 @@
 // the host loop and its copy took 205 ms of a handle's creation, this 0.1 ms.
 #pragma once
 
+#include "element_kernels.cuh"
 #include "kat_kernels.cuh"
-#include "kernels.cuh"
 
 namespace strut {
 
@@ -25,11 +25,30 @@ __global__ void init_history_kernel(const DevElem* __restrict__ elems, Geo g, Fi
     const DevSection& sd = g.secs[E.sec];
     const int nip = E.nip;
     int base = sd.geo_off;
-    for (int t = threadIdx.x; t < nip * sd.n_s2; t += blockDim.x)
-        init_s2(g.mats[g.m[base + t % sd.n_s2]], fs.s2 + E.s2_off + t, fs.s2_n);
+    for (int t = threadIdx.x; t < nip * sd.n_s2; t += blockDim.x) {
+        const DevMat& m = g.mats[g.m[base + t % sd.n_s2]];
+        double* F = fs.s2 + E.s2_off + t;
+        init_s2(m, F, fs.s2_n);
+        S2State c;
+        c.eps = F[0];
+        c.sig = F[fs.s2_n];
+        c.epsmin = F[3 * fs.s2_n];
+        c.epsmax = F[4 * fs.s2_n];
+        c.epspl = c.epss0 = c.sigs0 = c.epsr = c.sigr = 0.0;
+        c.kon = 0;
+        double* D = fs.s2d + 14ll * E.s2_off + t;
+        store_s2d(m, c, true, D, E.s2_blk);
+        store_s2d(m, c, false, D, E.s2_blk);
+    }
     base += sd.n_s2;
-    for (int t = threadIdx.x; t < nip * sd.n_c2; t += blockDim.x)
-        fs.c2[2 * fs.c2_n + E.c2_off + t] = g.mats[g.m[base + t % sd.n_c2]].k[C2K_EC0];
+    for (int t = threadIdx.x; t < nip * sd.n_c2; t += blockDim.x) {
+        const DevMat& m = g.mats[g.m[base + t % sd.n_c2]];
+        C2State c;
+        c.eps = c.sig = c.ecmin = c.dept = 0.0;
+        c.tan = m.k[C2K_EC0];
+        fs.c2[2 * fs.c2_n + E.c2_off + t] = c.tan;
+        store_c2d(m, c, fs.c2d + 5ll * E.c2_off + t, E.c2_blk);
+    }
     base += sd.n_c2;
     for (int t = threadIdx.x; t < nip * sd.n_s1; t += blockDim.x)
         fs.s1[2 * fs.s1_n + E.s1_off + t] = g.mats[g.m[base + t % sd.n_s1]].p[1];

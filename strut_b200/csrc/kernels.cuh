@@ -209,6 +209,10 @@ struct FiberState {
     long long s2_n;
     double* s1;
     long long s1_n;
+    // constants derived from the committed state, element blocks: field f of entry i of element e at
+    // (5 c2_off + f c2_blk + i) and (14 s2_off + f s2_blk + i)
+    double* c2d;
+    double* s2d;
     double* c1;  // Concrete01: eps, sig, tan, min strain, end strain, unloading slope
     long long c1_n;
 };

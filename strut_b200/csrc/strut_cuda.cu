@@ -1042,13 +1042,12 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             E.c1_blk = round4(E.nip * sd.n_c1);
             c1_total += E.c1_blk;
             h->max_nip = std::max(h->max_nip, E.nip);
-            // staged history (Concrete02 without dept) + derived constants (Concrete02 5, Steel02
-            // 14 doubles per fiber) + the section's fiber y + per-fiber stress and tangent of
-            // every point
+            // staged history (Concrete02 without dept, Steel02 strain and branch) + derived constants
+            // (Concrete02 5, Steel02 14 doubles per fiber) + the section's fiber y + per-fiber stress
+            // and tangent of every point
             const int n_tot = sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el;
-            const size_t smem = 8 * (size_t)(4 * E.c2_blk + 10 * E.s2_blk + 5 * E.s1_blk + 6 * E.c1_blk) +
+            const size_t smem = 8 * (size_t)(9 * E.c2_blk + 15 * E.s2_blk + 5 * E.s1_blk + 6 * E.c1_blk) +
                                 4 * (size_t)E.s2_blk +
-                                8 * (size_t)(5 * E.c2_blk + 14 * E.s2_blk) +
                                 8 * (size_t)((three_d ? 2 : 1) * ((n_tot + 1) & ~1) + 2 * E.nip * n_tot);
             h->elem_smem = std::max(h->elem_smem, smem);
             h->elem_fibers.push_back((long long)E.nip * (sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el));
@@ -1419,7 +1418,8 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         const long long c1n = round4((int)std::max<long long>(c1_total, 4));
         if ((rc = dzeros(&h->fs.c2, (size_t)(5 * c2n), al)) || (rc = dzeros(&h->fs.s2, (size_t)(10 * s2n), al)) ||
             (rc = dzeros(&h->fs.s2_kon, (size_t)s2n, al)) || (rc = dzeros(&h->fs.s1, (size_t)(5 * s1n), al)) ||
-            (rc = dzeros(&h->fs.c1, (size_t)(6 * c1n), al)))
+            (rc = dzeros(&h->fs.c1, (size_t)(6 * c1n), al)) || (rc = dzeros(&h->fs.c2d, (size_t)(5 * c2n), al)) ||
+            (rc = dzeros(&h->fs.s2d, (size_t)(14 * s2n), al)))
             return bail(rc);
         h->fs.c2_n = c2n;
         h->fs.s2_n = s2n;
