@@ -508,14 +508,26 @@ __device__ __forceinline__ void sum_phase(const DevSection& sd, int nip, const d
         const int g0 = b * cs, g1 = min(g0 + cs, n_tot);
         const double* f = fo + 2 * ip * n_tot;
         const int gm = min(g1, n_nl);
-#pragma unroll 4
-        for (int gg = g0; gg < gm; ++gg) {
-            const double fs = f[2 * gg], ks = f[2 * gg + 1], y = ys[gg];
-            a0 += fs;
-            a1 += -fs * y;
-            a2 += ks;
-            a3 += -ks * y;
-            a4 += ks * y * y;
+        // eight fibers at a time, loaded ahead of the additions (a remainder loop costs more)
+        for (int g8 = g0; g8 < gm; g8 += 8) {
+            double2 fk[8];
+            double y8[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int gg = min(g8 + u, gm - 1);
+                fk[u] = reinterpret_cast<const double2*>(f)[gg];
+                y8[u] = ys[gg];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (g8 + u < gm) {
+                    const double fs = fk[u].x, ks = fk[u].y, y = y8[u];
+                    a0 += fs;
+                    a1 += -fs * y;
+                    a2 += ks;
+                    a3 += -ks * y;
+                    a4 += ks * y * y;
+                }
         }
         for (int gg = max(g0, n_nl); gg < g1; ++gg) {
             const double fs = f[2 * gg], ks = f[2 * gg + 1], y = ys[gg];
@@ -578,9 +590,16 @@ __device__ __forceinline__ void lane_ordered_sums(double (*scr)[12], int nip, do
     __syncwarp();
 #pragma unroll
     for (int v = 0; v < NV; ++v) out[v] = 0.0;
-    for (int ip = 0; ip < nip; ++ip) {
+    if (nip == 5) {  // the usual rule, without a loop around the additions
 #pragma unroll
-        for (int v = 0; v < NV; ++v) out[v] += scr[ip][v];
+        for (int ip = 0; ip < 5; ++ip)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) out[v] += scr[ip][v];
+    } else {
+        for (int ip = 0; ip < nip; ++ip) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) out[v] += scr[ip][v];
+        }
     }
     __syncwarp();
 }
@@ -1588,54 +1607,59 @@ __global__ void __launch_bounds__(kTeamThreads) element_state_kernel(
             }
         }
     }
-    if (tid == 0) {
-        int fail = 0;
+    if (tid < 32) {
+        // warp 0: the state the element keeps, and its element state written by lanes
         if (!converged) {
-            for (int i = 0; i < 3; ++i) S.q[i] = S.acc_q[i];
-            for (int ip = 0; ip < nip; ++ip) {
-                S.vs_e[ip] = S.svs_e[ip];
-                S.vs_k[ip] = S.svs_k[ip];
+            if (tid < 3) S.q[tid] = S.acc_q[tid];
+            if (tid < nip) {
+                S.vs_e[tid] = S.svs_e[tid];
+                S.vs_k[tid] = S.svs_k[tid];
             }
+            __syncwarp();
         }
-        if (!S.best_ok) {
-            // _force_beam_column2d_initial_basic_tangent fallback
-            double F[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-            for (int ip = 0; ip < nip; ++ip) {
-                const double xi = E.xi[ip], wL = E.w[ip] * L;
-                flex_accum(F, wL, xi - 1.0, xi, sd.f00, sd.f01, sd.f11);
+        if (tid == 0) {
+            int fail = 0;
+            if (!S.best_ok) {
+                // _force_beam_column2d_initial_basic_tangent fallback
+                double F[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+                for (int ip = 0; ip < nip; ++ip) {
+                    const double xi = E.xi[ip], wL = E.w[ip] * L;
+                    flex_accum(F, wL, xi - 1.0, xi, sd.f00, sd.f01, sd.f11);
+                }
+                double k[9];
+                if (sd.init_valid && invert3(F, k)) {
+                    S.best[0] = S.q[0];
+                    S.best[1] = S.q[1];
+                    S.best[2] = S.q[2];
+                    for (int i = 0; i < 6; ++i) S.best[3 + i] = k[i];
+                    S.best[9] = k[8];
+                } else {
+                    fail = 1;
+                }
             }
-            double k[9];
-            if (sd.init_valid && invert3(F, k)) {
-                S.best[0] = S.q[0];
-                S.best[1] = S.q[1];
-                S.best[2] = S.q[2];
-                for (int i = 0; i < 6; ++i) S.best[3 + i] = k[i];
-                S.best[9] = k[8];
-            } else {
-                fail = 1;
-            }
-        }
-        S.flag = fail;
-        // element state: q, section deformations, accepted basic deformation
-        for (int i = 0; i < 3; ++i) {
-            estate[(size_t)e * kEStride + kEq + i] = S.q[i];
-            estate[(size_t)e * kEStride + kEv + i] = S.acc_v[i];
+            S.flag = fail;
         }
         double* es = estate + (size_t)e * kEStride;
-        for (int ip = 0; ip < nip; ++ip) {
-            es[kEe + ip] = S.vs_e[ip];
-            es[kEk + ip] = S.vs_k[ip];
-            es[kEcN + ip] = S.c_n[ip];
-            es[kEcM + ip] = S.c_m[ip];
-            es[kEc00 + ip] = S.c_f00[ip];
-            es[kEc01 + ip] = S.c_f01[ip];
-            es[kEc11 + ip] = S.c_f11[ip];
+        if (tid < 3) {
+            es[kEq + tid] = S.q[tid];
+            es[kEv + tid] = S.acc_v[tid];
         }
-        es[kEcv] = S.c_valid ? 1.0 : 0.0;
-        if (el.hard_flag && mode == ELEM_MODE_LIST) el.hard_flag[e] = ctl->fan ? S.hard : 0;
-        if (fslot >= 0) {
-            atomicAdd(&counters[6], 1ull);
-            atomicAdd(&el.fan_finished[cur], 1);  // the fanned element is resolved
+        if (tid < nip) {
+            es[kEe + tid] = S.vs_e[tid];
+            es[kEk + tid] = S.vs_k[tid];
+            es[kEcN + tid] = S.c_n[tid];
+            es[kEcM + tid] = S.c_m[tid];
+            es[kEc00 + tid] = S.c_f00[tid];
+            es[kEc01 + tid] = S.c_f01[tid];
+            es[kEc11 + tid] = S.c_f11[tid];
+        }
+        if (tid == 31) {
+            es[kEcv] = S.c_valid ? 1.0 : 0.0;
+            if (el.hard_flag && mode == ELEM_MODE_LIST) el.hard_flag[e] = ctl->fan ? S.hard : 0;
+            if (fslot >= 0) {
+                atomicAdd(&counters[6], 1ull);
+                atomicAdd(&el.fan_finished[cur], 1);  // the fanned element is resolved
+            }
         }
     }
     __syncthreads();
