@@ -1263,23 +1263,34 @@ __global__ void __launch_bounds__(kTeamThreads) element_state_kernel(
     double* ys = sv.tail;
     double* fo = ys + ((n_tot + 1) & ~1);
     int err = ELEM_ERR_NONE;
+    // (the element state's and the fiber y's loads go out before the copies are issued)
+    const double* es = estate + (size_t)e * kEStride;
+    double st[7];
+    if (tid < E.nip) {
+        st[0] = es[kEe + tid];
+        st[1] = es[kEk + tid];
+        st[2] = es[kEcN + tid];
+        st[3] = es[kEcM + tid];
+        st[4] = es[kEc00 + tid];
+        st[5] = es[kEc01 + tid];
+        st[6] = es[kEc11 + tid];
+    }
+    const double y0 = tid < n_tot ? __ldg(g.y + sd.geo_off + tid) : 0.0;
     const uint32_t stage_bytes = stage_issue(E, fs, smem_fib, &bar, sv);
     {
-        const double* es = estate + (size_t)e * kEStride;
         if (tid < E.nip) {
             const int ip = tid;
-            const double ve = es[kEe + ip], vk = es[kEk + ip];
-            S.vs_e[ip] = ve;
-            S.vs_k[ip] = vk;
+            S.vs_e[ip] = st[0];
+            S.vs_k[ip] = st[1];
             if (E.type == 2) {  // the accepted section deformations start as the element's
-                S.svs_e[ip] = ve;
-                S.svs_k[ip] = vk;
+                S.svs_e[ip] = st[0];
+                S.svs_k[ip] = st[1];
             }
-            S.c_n[ip] = es[kEcN + ip];
-            S.c_m[ip] = es[kEcM + ip];
-            S.c_f00[ip] = es[kEc00 + ip];
-            S.c_f01[ip] = es[kEc01 + ip];
-            S.c_f11[ip] = es[kEc11 + ip];
+            S.c_n[ip] = st[2];
+            S.c_m[ip] = st[3];
+            S.c_f00[ip] = st[4];
+            S.c_f01[ip] = st[5];
+            S.c_f11[ip] = st[6];
         } else if (tid == 32) {
             // the displacements in the element's frame and (forceBeamColumn2d) the basic
             // deformations, the accepted state and the increment still to apply
@@ -1319,7 +1330,8 @@ __global__ void __launch_bounds__(kTeamThreads) element_state_kernel(
             }
         }
     }
-    for (int gg = tid; gg < n_tot; gg += blockDim.x) ys[gg] = __ldg(g.y + sd.geo_off + gg);
+    if (tid < n_tot) ys[tid] = y0;
+    for (int gg = tid + blockDim.x; gg < n_tot; gg += blockDim.x) ys[gg] = __ldg(g.y + sd.geo_off + gg);
     const bool staged = stage_wait(stage_bytes, &bar, phase, &err);  // a CTA barrier when copies ran
     if (!stage_bytes) __syncthreads();
     if (!staged) {
@@ -1682,15 +1694,39 @@ __global__ void __launch_bounds__(kTeamThreads) element_state_kernel(
                    av[2] * (kb[6] * bv[0] + kb[7] * bv[1] + kb[8] * bv[2]);
     }
     __syncthreads();
-    if (tid == 0) {
-        const double q0 = S.best[0], q1 = S.best[1], q2 = S.best[2];
+    if (tid < 32) {
+        // warp 0: PDelta terms and the rotation to global axes (k_to_global), six lanes a row, then a
+        // column each
+        const double c = E.c, s = E.s;
         if (E.geom == 1) {
-            const double ql = q0 * inv_L;
-            S.k[1 * 6 + 1] += ql;
-            S.k[4 * 6 + 4] += ql;
-            S.k[1 * 6 + 4] -= ql;
-            S.k[4 * 6 + 1] -= ql;
+            if (tid == 0) {
+                const double ql = S.best[0] * inv_L;
+                S.k[1 * 6 + 1] += ql;
+                S.k[4 * 6 + 4] += ql;
+                S.k[1 * 6 + 4] -= ql;
+                S.k[4 * 6 + 1] -= ql;
+            }
+            __syncwarp();
         }
+        if (tid < 6) {
+            double* k = S.k + 6 * tid;
+            const double k0 = k[0], k1 = k[1], k3 = k[3], k4 = k[4];
+            k[0] = c * k0 - s * k1;
+            k[1] = s * k0 + c * k1;
+            k[3] = c * k3 - s * k4;
+            k[4] = s * k3 + c * k4;
+        }
+        __syncwarp();
+        if (tid < 6) {
+            double* k = S.k + tid;
+            const double a0 = k[0], b0 = k[6], a1 = k[18], b1 = k[24];
+            k[0] = c * a0 - s * b0;
+            k[6] = s * a0 + c * b0;
+            k[18] = c * a1 - s * b1;
+            k[24] = s * a1 + c * b1;
+        }
+    } else if (tid == 32) {
+        const double q0 = S.best[0], q1 = S.best[1], q2 = S.best[2];
         S.f[0] = -q0 + 0.0;
         S.f[1] = (q1 + q2) * inv_L + 0.0;
         S.f[2] = q1;
@@ -1702,8 +1738,8 @@ __global__ void __launch_bounds__(kTeamThreads) element_state_kernel(
             S.f[1] += ps;
             S.f[4] -= ps;
         }
-        k_to_global(S.k, E.c, E.s);
         f_to_global(S.f, E.c, E.s);
+    } else if (tid == 64) {
         atomicAdd(&counters[3], (unsigned long long)E.io_bytes);
         atomicAdd(&counters[0], (unsigned long long)S.local_iters);
         atomicMax(&counters[5], (unsigned long long)S.local_iters);
