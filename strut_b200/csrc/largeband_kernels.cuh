@@ -9,8 +9,8 @@
 //                          partial pivoting, panel width kPanel, the right-hand side carried as
 //                          one more column.  CTA 0 factors the panel in shared memory; every CTA
 //                          then takes column tiles of the trailing block (the panel's row
-//                          interchanges, then the eliminations in column order).  Two bounded
-//                          grid barriers per panel.
+//                          interchanges, then the eliminations in column order).  Two one-way
+//                          signals per panel, each waited for a bounded number of polls.
 //   large_solve_kernel     one CTA per instance: blocked back substitution through U, then the
 //                          displacement update and the convergence test shared with the
 //                          shared-memory path.
@@ -35,56 +35,60 @@ namespace strut {
 
 constexpr int kPanel = 32;         // panel width of the blocked band LU
 constexpr int kLargeThreads = 384; // threads of a factorisation CTA (one per panel row)
-// The variant for wider bands: 16-column panels and 640 threads (the panel rows' registers halve,
-// so more rows fit a CTA).  Every entry receives the same subtractions in the same column order
+// The variant for wider bands: 16-column panels and 640 threads (the panel rows halve,
+// so more of them fit a CTA's shared memory).  Every entry receives the same subtractions in the same column order
 // with either variant, so their results are the same bit for bit.
 constexpr int kPanelWide = 16;
 constexpr int kLargeThreadsWide = 640;
 constexpr int kSolveThreads = 1024;
 
 constexpr int kColTile = 16;       // trailing-update columns per tile
+// The variant for half bands up to 96 (15 nodes a floor): 128 threads, so every warp can look through
+// the whole column by itself and a panel column needs one barrier of four warps instead of two of
+// twelve; 8-column tiles, which double the CTAs of the trailing update.
+constexpr int kLargeThreadsNarrow = 128;
+constexpr int kColTileNarrow = 8;
 enum { LSTAT_OK = 0, LSTAT_SINGULAR = 2, LSTAT_CONVERGED = 7, LSTAT_IDLE = -1 };
 
 struct GridBarrier {
-    unsigned int count;
-    unsigned int gen;
+    unsigned int done;   // CTAs other than 0 that are through with a panel, over all panels
+    unsigned int panel;  // panels that CTA 0 has published, times two, plus one if it is singular
     int err;
-    int pad;
     int limit;  // polls a waiting CTA makes before it gives up (strut_gpu_set_wait_limit)
-    int pad2;
 };
 
 constexpr int kBarrierPolls = 1 << 22;
 
-// Grid-wide barrier of a cooperative launch.  Thread 0 of each CTA arrives; the last arrival
-// resets the count and advances the generation; the others wait for the generation to move,
-// for a bounded number of polls (gb->limit), after which the barrier records an error and every
-// CTA stops.
-__device__ __forceinline__ bool grid_barrier(GridBarrier* gb, unsigned int& gen) {
-    __syncthreads();
+// The CTAs of the cooperative factorisation hand each other two words, both reset before each
+// launch: CTA 0 publishes a panel, the others count themselves off when they are through with its
+// columns and go on to wait for the next; only CTA 0 waits for the count.  One way each, where a
+// barrier of all costs two trips through L2 for the arrival and the reset and one for the release
+// (2,700 cycles a barrier).  A wait makes gb->limit polls at most, then it records an error and
+// the CTA stops; the others run out in turn.
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Thread 0 polls until ready(word); the CTA gets the word.  False once the wait was given up.
+template <class Ready>
+__device__ __forceinline__ bool await_word(GridBarrier* gb, const unsigned int* p, unsigned int* s_word, Ready ready) {
     int ok = 1;
     if (threadIdx.x == 0) {
-        const unsigned int g = gen;
-        __threadfence();
-        const unsigned int arrived = atomicAdd(&gb->count, 1u) + 1u;
-        if (arrived == gridDim.x) {
-            atomicExch(&gb->count, 0u);
-            __threadfence();
-            atomicAdd(&gb->gen, 1u);
-        } else {
-            int polls = 0;
-            const int limit = *(volatile int*)&gb->limit;
-            while (atomicAdd(&gb->gen, 0u) == g) {
-                if (++polls > limit || atomicAdd(&gb->err, 0) != 0) {
-                    atomicExch(&gb->err, 1);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
+        const int limit = *(volatile int*)&gb->limit;
+        int polls = 0;
+        unsigned int v = ld_acquire(p);
+        while (!ready(v)) {
+            if (++polls > limit || ((polls & 63) == 0 && *(volatile int*)&gb->err != 0)) {
+                atomicExch(&gb->err, 1);
+                ok = 0;
+                break;
             }
+            v = ld_acquire(p);
         }
         __threadfence();
-        gen = g + 1u;
+        *s_word = v;
     }
     return __syncthreads_and(ok) != 0;
 }
@@ -109,7 +113,8 @@ __global__ void __launch_bounds__(256) large_assemble_kernel(const DevInst* __re
     const int lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // the factorisation that follows starts from a clean barrier
-        gb->count = 0u;
+        gb->done = 0u;
+        gb->panel = 0u;
         gb->err = 0;
     }
     if (warp_g >= total_rows) return;
@@ -240,7 +245,8 @@ __global__ void large_load_exported_kernel(const DevInst* __restrict__ insts, In
                                            const int* __restrict__ large_list, int n_large,
                                            GridBarrier* gb, double* __restrict__ wbuf) {
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-        gb->count = 0u;
+        gb->done = 0u;
+        gb->panel = 0u;
         gb->err = 0;
     }
     const int li = blockIdx.y;
@@ -259,24 +265,29 @@ __global__ void large_load_exported_kernel(const DevInst* __restrict__ insts, In
 
 // Shared memory of large_factor_kernel: the panel's unit lower triangle L11
 // (kPanel x (kPanel + 1)); CTA 0's panel rows (kLargeThreads x (kPanel + 1)), whose space the
-// column slab of the trailing phase ((kPanel + bw) x (kColTile + 2)) reuses; the row at the
-// diagonal (two, by column parity) and the row that replaces it; the panel's row permutation.
+// column slab of the trailing phase ((kPanel + bw) x (kColTile + 2)) reuses; four rows of U; four
+// columns by place (two sets, by column parity); the panel's row permutation.
 // Row stride of the panel-row buffer, which the slab (stride kColTile + 2) reuses.
 __host__ __device__ constexpr int large_row_stride(int panel) {
     return panel + 1 > kColTile + 2 ? panel + 1 : kColTile + 2;
 }
+__host__ __device__ constexpr int large_col_tile(int threads) {
+    return threads == kLargeThreadsNarrow ? kColTileNarrow : kColTile;
+}
 __host__ __device__ inline size_t large_factor_smem(int panel, int threads) {
-    return sizeof(double) * ((size_t)panel * (panel + 1) + (size_t)threads * large_row_stride(panel) + 3 * panel) +
+    return sizeof(double) * ((size_t)panel * (panel + 1) + (size_t)threads * large_row_stride(panel) + 4 * panel +
+                             8 * (size_t)threads) +
            sizeof(int) * (size_t)threads;
 }
 
 // Column tiles of the trailing update of one panel (+1: the right-hand side): the CTAs a
 // factorisation can keep busy.
-__host__ __device__ inline int large_factor_tiles(int bw) {
-    return (2 * bw + kColTile - 1) / kColTile + 1;
+__host__ __device__ inline int large_factor_tiles(int bw, int threads) {
+    return (2 * bw + large_col_tile(threads) - 1) / large_col_tile(threads) + 1;
 }
 
 // Largest half-band each variant takes: one thread per panel row.
+constexpr int kLargeMaxBwNarrow = kLargeThreadsNarrow - kPanel;
 constexpr int kLargeMaxBw = kLargeThreads - kPanel;
 constexpr int kLargeMaxBwWide = kLargeThreadsWide - kPanelWide;
 
@@ -298,12 +309,17 @@ __device__ __forceinline__ void warp_argmax_first(double& v, int& idx) {
 // (column-major, leading dimension kLargeThreads) / lperm: the factored panel and the row
 // permutation of its interchanges, from CTA 0 to the others.
 //
-// Per panel: CTA 0 factors the panel columns with one thread per panel row, the row in
-// registers, four columns per rolled step (the finished columns go to shared memory and the
-// row shifts left).  Per column the row at the diagonal publishes itself as the pivot row and
-// one block vote asks whether any row below beats it strictly; only then the full search for the
-// first largest entry runs and the two rows are exchanged whole (multipliers included).  Grid
-// barrier; every CTA takes column tiles of the trailing block: loads them with the panel's row
+// Per panel: CTA 0 factors the panel columns with one thread per panel row, the row in shared
+// memory and four of its columns in registers.  A column is one chain of latencies (offer the
+// entries by place, barrier, pivot and its reciprocal beside the vote, multiplier, the rest of the
+// four columns), so it has no branch but the vote's: only where a row beats the diagonal
+// strictly, or the diagonal is small, the search for the first largest entry runs, and an
+// interchange swaps the places of two rows, not the rows.  After four columns the pivot rows
+// behind them are formed by one warp, lane = column, and every row takes its four updates an
+// entry in the columns' order.  Rows exchanged whole, a vote of twelve warps and a division a
+// column took 30,200 cycles a panel of 32 columns (n = 936, half band 83), this 17,500; the
+// factorisation with its loads and signals 63,200 cycles a panel, now 34,200.  CTA 0
+// publishes the panel; every CTA takes column tiles of the trailing block: loads them with the panel's row
 // permutation applied, solves the panel rows against the unit lower L11 on the warps (lane =
 // row), subtracts L21 U12 from the rows below entry by entry in column order (one thread per
 // row, the row's multipliers in registers); grid barrier.
@@ -312,24 +328,38 @@ __global__ void __launch_bounds__(THREADS) large_factor_kernel(
     const DevInst* __restrict__ insts, InstArrays A, const int* __restrict__ large_list,
     int n_large, int mode, GridBarrier* gb, double* wbuf, double* lpan, int* lperm) {
     extern __shared__ __align__(16) double smem_lf[];
-    __shared__ int s_flag[2];
-    __shared__ int s_piv[PANEL];
+    __shared__ int s_flag[1];
     __shared__ double red[32];
-    __shared__ int red_r[32];
     constexpr int kPs = PANEL + 1;     // row stride of L11
     constexpr int kRs = large_row_stride(PANEL);  // row stride of the panel rows and the slab
-    constexpr int kSs = kColTile + 2;   // row stride of the slab (even: 16-byte rows)
+    constexpr int CT = large_col_tile(THREADS);
+    constexpr bool kNarrow = THREADS == kLargeThreadsNarrow;
+    constexpr int kFly = kNarrow ? 8 : 4;  // loads in flight per thread
+    constexpr int kSs = CT + 2;   // row stride of the slab (even: 16-byte rows)
     constexpr int kLd = THREADS;  // leading dimension of lpan
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
     const int nwarps = nt >> 5;
     double* L11 = smem_lf;                              // PANEL x kPs
     double* Pout = L11 + PANEL * kPs;                  // panel rows (CTA 0), THREADS x kRs
     double* S = Pout;                                   // slab of the trailing phase, pr x kSs
-    double* prow2 = Pout + (size_t)THREADS * kRs;       // row at the diagonal, by column parity
-    double* crow = prow2 + 2 * PANEL;                  // the row that replaces it
-    int* s_perm = (int*)(crow + PANEL);                // panel row -> original row
-    unsigned int gen = 0;
-    if (tid == 0) gen = atomicAdd(&gb->gen, 0u);
+    double* ublk = Pout + (size_t)THREADS * kRs;        // four rows of U, PANEL x 4
+    double* colb = ublk + 4 * PANEL;                    // four columns by place, by column parity
+    int* s_perm = (int*)(colb + 8 * THREADS);           // panel row -> original row
+    __shared__ unsigned int s_word;
+    unsigned int panels = 0;  // published so far, over all instances
+    // CTA 0 waits for the others to be through with the panel, the others say that they are
+    auto finish = [&]() -> bool {
+        if (blockIdx.x == 0) {
+            const unsigned int all = panels * (gridDim.x - 1);
+            return await_word(gb, &gb->done, &s_word, [=](unsigned int v) { return v == all; });
+        }
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            atomicAdd(&gb->done, 1u);
+        }
+        return true;
+    };
     for (int li = 0; li < n_large; ++li) {
         const int inst = large_list[li];
         const DevInst& I = insts[inst];
@@ -364,140 +394,177 @@ __global__ void __launch_bounds__(THREADS) large_factor_kernel(
             const bool own = r < pr;
             if (blockIdx.x == 0) {
                 // ---- panel: rows k0..r1, columns k0..k0+kb-1 (rows loaded coalesced, lane = column)
-                for (int rb = wid; rb < pr; rb += 4 * nwarps) {
-                    double v[4];  // four rows in flight per warp
+                for (int rb = wid; rb < pr; rb += 2 * kFly * nwarps) {
+                    double v[2 * kFly];  // rows in flight per warp
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
+                    for (int m = 0; m < 2 * kFly; ++m) {
                         const int rr = rb + m * nwarps;
                         const int d = lane - rr;
                         v[m] = (rr < pr && lane < kb && d >= -bw && d <= 2 * bw) ? B[lslot(lrw, bw, k0 + rr, k0 + lane)]
                                                                                  : 0.0;
                     }
 #pragma unroll
-                    for (int m = 0; m < 4; ++m)
+                    for (int m = 0; m < 2 * kFly; ++m)
                         if (rb + m * nwarps < pr && lane < PANEL) Pout[(rb + m * nwarps) * kRs + lane] = v[m];
                 }
-                if (own) s_perm[r] = r;
                 if (tid == 0) s_flag[0] = LSTAT_OK;
                 __syncthreads();
-                double a[PANEL];  // a[q] = column c0 + q of this thread's row
-#pragma unroll
-                for (int q = 0; q < PANEL; ++q) a[q] = own ? Pout[r * kRs + q] : 0.0;
                 bool failed = false;
-                for (int c0 = 0; c0 < kb; c0 += 4) {
+                int pos = r;  // the row's place; interchanges move places, not rows
+                double* row = Pout + r * kRs;
+                for (int c0 = 0; c0 < kb && !failed; c0 += 4) {
+                    // One column: no branch but the vote's, which takes the rows in which the diagonal
+                    // is beaten or small out of the way.  Rows past the band hold zeros, as do the
+                    // places past the panel; rows that are done offer a zero and keep their entries.
+                    double a[4];  // a[q] = column c + q of this thread's row
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) {
-                        const int c = c0 + cc;
-                        if (c < kb && !failed) {
-                            const int last = min(pr - 1, c + bw);  // rows of column k0+c in the band
-                            const bool act = own && r > c && r <= last;
-                            // double buffered: a slow thread may still read the previous one
-                            double* prow = prow2 + (c & 1) * PANEL;
-                            if (r == c) {
+                    for (int q = 0; q < 4; ++q) a[q] = own ? row[c0 + q] : 0.0;
+                    const int ce = min(kb, c0 + 4);
+#pragma unroll 1
+                    for (int c = c0; c < ce; ++c) {
+                        // double buffered: a slow thread may still read the previous one
+                        double* cb = colb + (c & 1) * 4 * THREADS;
+                        const double offer = pos >= c ? a[0] : 0.0;
+                        cb[pos] = offer;
 #pragma unroll
-                                for (int q = 0; q < PANEL; ++q) prow[q] = a[q];
-                            }
-                            __syncthreads();
-                            // the reference's strict '>' scan keeps the diagonal unless a row
-                            // below beats it
-                            const double dabs = fabs(prow[cc]);
-                            const int any = __syncthreads_or(act && fabs(a[cc]) > dabs);
-                            const double* pivrow = prow;
-                            int p = c;
-                            if (any || dabs <= 1.0e-14) {
-                                double bv = (own && r >= c && r <= last) ? fabs(a[cc]) : -1.0;
-                                int br = r;
-                                warp_argmax_first(bv, br);
-                                if (lane == 0) {
-                                    red[wid] = bv;
-                                    red_r[wid] = br;
-                                }
-                                __syncthreads();
-                                double pv = lane < nwarps ? red[lane] : -2.0;
-                                p = lane < nwarps ? red_r[lane] : 0x7fffffff;
-                                warp_argmax_first(pv, p);
-                                if (pv <= 1.0e-14) {
-                                    failed = true;
-                                    if (tid == 0) s_flag[0] = LSTAT_SINGULAR;
-                                } else if (p != c) {
-                                    // whole rows, multipliers included, so that the trailing
-                                    // columns can take all interchanges first and the
-                                    // eliminations after
-                                    pivoted = 1;
-                                    if (r == p) {
+                        for (int q = 1; q < 4; ++q) cb[q * THREADS + pos] = a[q];
+                        __syncthreads();
+                        double u[4];
 #pragma unroll
-                                        for (int q = 0; q < PANEL; ++q) crow[q] = a[q];
-                                    }
-                                    if (tid == 0) {
-                                        const int o = s_perm[c];
-                                        s_perm[c] = s_perm[p];
-                                        s_perm[p] = o;
-                                    }
-                                    if (wid == 0 && lane < c0) {
-                                        // finished columns of earlier steps
-                                        const double t0 = Pout[c * kRs + lane];
-                                        Pout[c * kRs + lane] = Pout[p * kRs + lane];
-                                        Pout[p * kRs + lane] = t0;
-                                    }
-                                    __syncthreads();
-                                    if (r == c) {
+                        for (int q = 0; q < 4; ++q) u[q] = cb[q * THREADS + c];
+                        // the reference's strict '>' scan keeps the diagonal unless a row below
+                        // beats it, then takes the first largest
+                        const double dabs = fabs(u[0]);
+                        bool rare = dabs <= 1.0e-14;
+                        if constexpr (kNarrow) {
 #pragma unroll
-                                        for (int q = 0; q < PANEL; ++q) a[q] = crow[q];
-                                    } else if (r == p) {
-#pragma unroll
-                                        for (int q = 0; q < PANEL; ++q) a[q] = prow[q];
-                                    }
-                                    pivrow = crow;
+                            for (int m = 0; m < THREADS / 32; ++m) rare |= fabs(cb[lane + 32 * m]) > dabs;
+                            rare = __any_sync(0xffffffffu, rare);
+                        } else {
+                            rare = __syncthreads_or(rare || fabs(offer) > dabs);
+                        }
+                        double rpiv = recip(u[0]);  // beside the vote
+                        if (rare) {
+                            // a NaN is no candidate: every thread has to find the same row
+                            double pv = -1.0;
+                            int p = 0x7fffffff;
+                            for (int rr = c + lane; rr < pr; rr += 32) {
+                                const double v = fabs(cb[rr]);
+                                if (v > pv) {
+                                    pv = v;
+                                    p = rr;
                                 }
                             }
-                            if (!failed) {
-                                if (act) {
-                                    const double f = a[cc] / pivrow[cc];
-                                    a[cc] = f;
+                            warp_argmax_first(pv, p);
+                            if (pv <= 1.0e-14) {
+                                failed = true;
+                                if (tid == 0) s_flag[0] = LSTAT_SINGULAR;
+                                break;
+                            }
+                            if (p != c) {
+                                pivoted = 1;
 #pragma unroll
-                                    for (int q = cc + 1; q < PANEL; ++q)
-                                        if (c0 + q < kb) a[q] = fma(-f, pivrow[q], a[q]);
+                                for (int q = 0; q < 4; ++q) u[q] = cb[q * THREADS + p];
+                                rpiv = recip(u[0]);
+                                if (pos == c) pos = p;
+                                else if (pos == p) pos = c;
+                            }
+                        }
+                        const bool below = pos > c;
+                        const double f = quot(a[0], u[0], rpiv);
+                        a[0] = below ? f : a[0];
+                        row[c] = a[0];
+                        if (pos == c) s_perm[c] = r;
+#pragma unroll
+                        for (int q = 1; q < 4; ++q) {
+                            const double t = fma(-f, u[q], a[q]);
+                            a[q - 1] = below ? t : a[q];
+                        }
+                    }
+                    if (c0 + 4 < kb && !failed) {
+                        // the four pivot rows behind these columns, then four updates an entry,
+                        // in the columns' order
+                        __syncthreads();
+                        if (wid == 0 && lane >= c0 + 4 && lane < PANEL) {
+                            double* r0 = Pout + s_perm[c0] * kRs;
+                            double* r1 = Pout + s_perm[c0 + 1] * kRs;
+                            double* r2 = Pout + s_perm[c0 + 2] * kRs;
+                            double* r3 = Pout + s_perm[c0 + 3] * kRs;
+                            const double u0 = r0[lane];
+                            const double u1 = fma(-r1[c0], u0, r1[lane]);
+                            const double u2 = fma(-r2[c0 + 1], u1, fma(-r2[c0], u0, r2[lane]));
+                            const double u3 =
+                                fma(-r3[c0 + 2], u2, fma(-r3[c0 + 1], u1, fma(-r3[c0], u0, r3[lane])));
+                            r1[lane] = u1;
+                            r2[lane] = u2;
+                            r3[lane] = u3;
+                            double2* to = reinterpret_cast<double2*>(ublk + 4 * lane);
+                            to[0] = make_double2(u0, u1);
+                            to[1] = make_double2(u2, u3);
+                        }
+                        __syncthreads();
+                        if (own && pos >= c0 + 4 && pos <= c0 + 3 + bw) {
+                            double f[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) f[k] = row[c0 + k];
+#pragma unroll 2
+                            for (int q = c0 + 4; q < kb; q += 4) {
+                                double x[4];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) x[j] = row[q + j];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const double2* u = reinterpret_cast<const double2*>(ublk + 4 * (q + j));
+                                    const double2 lo = u[0], hi = u[1];
+                                    x[j] = fma(-f[0], lo.x, x[j]);
+                                    x[j] = fma(-f[1], lo.y, x[j]);
+                                    x[j] = fma(-f[2], hi.x, x[j]);
+                                    x[j] = fma(-f[3], hi.y, x[j]);
                                 }
-                                if (tid == 0) s_piv[c] = p;
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) row[q + j] = x[j];
                             }
                         }
                     }
-                    // columns c0 .. c0+3 are final: keep them, shift the row left by four
-                    if (own) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            if (c0 + q < PANEL) Pout[r * kRs + c0 + q] = a[q];
-                    }
-#pragma unroll
-                    for (int q = 0; q < PANEL; ++q) a[q] = q + 4 < PANEL ? a[q + 4] : 0.0;
                 }
+                if (own && pos >= kb) s_perm[pos] = r;
                 __syncthreads();
                 if (s_flag[0] == LSTAT_OK) {
-                    for (int t = tid; t < kb * pr; t += nt) {
-                        const int q = t / pr, rr = t - q * pr;
-                        lpan[q * kLd + rr] = Pout[rr * kRs + q];
+                    // thread = place in the panel
+                    if (own) {
+                        const double* placed = Pout + s_perm[r] * kRs;
+#pragma unroll 8
+                        for (int q = 0; q < kb; ++q) lpan[q * kLd + r] = placed[q];
+                        lperm[r] = s_perm[r];
                     }
                     for (int rr = wid; rr < kb; rr += nwarps)
-                        if (lane >= rr && lane < kb) B[lslot(lrw, bw, k0 + rr, k0 + lane)] = Pout[rr * kRs + lane];
-                    if (own) lperm[r] = s_perm[r];
+                        if (lane >= rr && lane < kb)
+                            B[lslot(lrw, bw, k0 + rr, k0 + lane)] = Pout[s_perm[rr] * kRs + lane];
                 }
+                __syncthreads();
+                ++panels;
+                result = s_flag[0];
                 if (tid == 0) {
-                    A.lstatus[li] = s_flag[0];
-                    // publish the panel result to the other CTAs through gb->pad
-                    atomicExch(&gb->pad, s_flag[0]);
+                    A.lstatus[li] = result;
+                    __threadfence();
+                    atomicExch(&gb->panel, 2 * panels + (result != LSTAT_OK ? 1 : 0));
                 }
+            } else {
+                ++panels;
+                const unsigned int want = panels;
+                if (!await_word(gb, &gb->panel, &s_word, [=](unsigned int v) { return (v >> 1) == want; })) return;
+                result = s_word & 1u ? LSTAT_SINGULAR : LSTAT_OK;
             }
-            if (!grid_barrier(gb, gen)) return;
-            if (tid == 0) s_flag[1] = atomicAdd(&gb->pad, 0);
-            __syncthreads();
-            result = s_flag[1];
-            if (result != LSTAT_OK) break;
-            // ---- trailing columns k0+kb .. c1 in tiles of kColTile, and the right-hand side
+            if (result != LSTAT_OK) {
+                if (!finish()) return;
+                break;
+            }
+            // ---- trailing columns k0+kb .. c1 in tiles of CT, and the right-hand side
             const int j_first = k0 + kb;
             const int ncols = c1 - j_first + 1;
-            const int ntiles = (ncols > 0 ? (ncols + kColTile - 1) / kColTile : 0) + 1;
+            const int ntiles = (ncols > 0 ? (ncols + CT - 1) / CT : 0) + 1;
             if (blockIdx.x >= ntiles) {
-                if (!grid_barrier(gb, gen)) return;
+                if (!finish()) return;
                 continue;
             }
             // this thread's panel row: its multipliers (L21, or L11 for the first kb rows)
@@ -513,79 +580,92 @@ __global__ void __launch_bounds__(THREADS) large_factor_kernel(
             }
             for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
                 const bool rhs = tile == ntiles - 1;
-                const int j0 = j_first + tile * kColTile;
-                const int ct = rhs ? 1 : min(kColTile, c1 - j0 + 1);
+                const int j0 = j_first + tile * CT;
+                const int ct = rhs ? 1 : min(CT, c1 - j0 + 1);
                 __syncthreads();
-                for (int t0 = tid; t0 < pr * ct; t0 += 4 * nt) {
-                    double v[4];  // four loads in flight per thread
+                if (rhs) {
+                    if (own) S[r * kSs] = w[k0 + s_perm[r]];
+                } else {
+                    for (int t0 = tid; t0 < pr * CT; t0 += kFly * nt) {
+                        double v[kFly];
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const int t = t0 + m * nt;
-                        v[m] = 0.0;
-                        if (t < pr * ct) {
-                            const int rr = t / ct, q = t - rr * ct;
-                            const int src = k0 + s_perm[rr];
-                            const int d = j0 + q - src;
-                            if (rhs) v[m] = w[src];
-                            else if (d >= -bw && d <= 2 * bw) v[m] = B[lslot(lrw, bw, src, j0 + q)];
+                        for (int m = 0; m < kFly; ++m) {
+                            const int t = t0 + m * nt, rr = t / CT, q = t % CT;
+                            v[m] = 0.0;
+                            if (rr < pr && q < ct) {
+                                const int src = k0 + s_perm[rr];
+                                const int d = j0 + q - src;
+                                if (d >= -bw && d <= 2 * bw) v[m] = B[lslot(lrw, bw, src, j0 + q)];
+                            }
                         }
-                    }
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const int t = t0 + m * nt;
-                        if (t < pr * ct) {
-                            const int rr = t / ct;
-                            S[rr * kSs + (t - rr * ct)] = v[m];
+                        for (int m = 0; m < kFly; ++m) {
+                            const int t = t0 + m * nt, rr = t / CT, q = t % CT;
+                            if (rr < pr) S[rr * kSs + q] = v[m];
                         }
                     }
                 }
                 __syncthreads();
-                // U12 = L11^-1 (P A12): one warp per column, lane = panel row
-                for (int q = wid; q < ct; q += nwarps) {
+                // U12 = L11^-1 (P A12): lane = panel row, two columns a warp, whose chains of
+                // shuffle and FMA (one step a panel column) overlap
+                for (int q = wid; q < ct; q += 2 * nwarps) {
+                    const int q1 = q + nwarps;
                     double v = lane < kb ? S[lane * kSs + q] : 0.0;
+                    double v1 = lane < kb && q1 < ct ? S[lane * kSs + q1] : 0.0;
+#pragma unroll 4
                     for (int sc = 0; sc + 1 < kb; ++sc) {
                         const double u = __shfl_sync(0xffffffffu, v, sc);
-                        if (lane > sc && lane < kb) v = fma(-L11[lane * kPs + sc], u, v);
+                        const double u1 = __shfl_sync(0xffffffffu, v1, sc);
+                        if (lane > sc && lane < kb) {
+                            const double f = -L11[lane * kPs + sc];
+                            v = fma(f, u, v);
+                            v1 = fma(f, u1, v1);
+                        }
                     }
                     if (lane < kb) S[lane * kSs + q] = v;
+                    if (lane < kb && q1 < ct) S[lane * kSs + q1] = v1;
                 }
                 __syncthreads();
                 // A22 -= L21 U12 entry by entry, column order; one thread per row
-                double v[kColTile];
+                double v[CT];
                 if (own && r >= kb) {
 #pragma unroll
-                    for (int q = 0; q < kColTile; ++q) v[q] = S[r * kSs + q];
+                    for (int q = 0; q < CT; ++q) v[q] = S[r * kSs + q];
+                    auto step = [&](int sc) {
+                        const double f = lrow[sc];
 #pragma unroll
-                    for (int sc = 0; sc < PANEL; ++sc) {
-                        if (sc < kb) {
-                            const double f = lrow[sc];
-#pragma unroll
-                            for (int q2 = 0; q2 < kColTile / 2; ++q2) {
-                                const double2 u = reinterpret_cast<const double2*>(S + sc * kSs)[q2];
-                                v[2 * q2] = fma(-f, u.x, v[2 * q2]);
-                                v[2 * q2 + 1] = fma(-f, u.y, v[2 * q2 + 1]);
-                            }
+                        for (int q2 = 0; q2 < CT / 2; ++q2) {
+                            const double2 u = reinterpret_cast<const double2*>(S + sc * kSs)[q2];
+                            v[2 * q2] = fma(-f, u.x, v[2 * q2]);
+                            v[2 * q2 + 1] = fma(-f, u.y, v[2 * q2 + 1]);
                         }
+                    };
+                    if (kNarrow && kb == PANEL) {  // without a test a step, so that loads run ahead
+#pragma unroll
+                        for (int sc = 0; sc < PANEL; ++sc) step(sc);
+                    } else {
+#pragma unroll
+                        for (int sc = 0; sc < PANEL; ++sc)
+                            if (sc < kb) step(sc);
                     }
                 }
                 __syncthreads();
                 if (own && r >= kb) {
 #pragma unroll
-                    for (int q = 0; q < kColTile; ++q) S[r * kSs + q] = v[q];
+                    for (int q = 0; q < CT; ++q) S[r * kSs + q] = v[q];
                 }
                 __syncthreads();
-                for (int t = tid; t < pr * ct; t += nt) {
-                    const int rr = t / ct, q = t - rr * ct;
-                    const int i = k0 + rr;
-                    if (rhs) {
-                        w[i] = S[rr * kSs];
-                    } else {
+                if (rhs) {
+                    if (own) w[k0 + r] = S[r * kSs];
+                } else {
+                    for (int t = tid; t < pr * CT; t += nt) {
+                        const int rr = t / CT, q = t % CT, i = k0 + rr;
                         const int d = j0 + q - i;
-                        if (d >= -bw && d <= 2 * bw) B[lslot(lrw, bw, i, j0 + q)] = S[rr * kSs + q];
+                        if (q < ct && d >= -bw && d <= 2 * bw) B[lslot(lrw, bw, i, j0 + q)] = S[rr * kSs + q];
                     }
                 }
             }
-            if (!grid_barrier(gb, gen)) return;
+            if (!finish()) return;
         }
         if (blockIdx.x == 0 && tid == 0 && pivoted && result == LSTAT_OK && A.fallbacks) A.fallbacks[inst] += 1;
     }

@@ -301,7 +301,8 @@ struct StrutHandle {
     int* d_large_rowbase = nullptr;
     GridBarrier* d_gb = nullptr;
     double* d_wbuf = nullptr;
-    int lfactor_wide = 0;      // the 16-column / 640-thread factorisation (half bands beyond 352)
+    const void* lfactor = nullptr;  // large_factor_kernel for the widest band, its threads
+    int lfactor_threads = 0;
     double* d_lpan = nullptr;  // factored panel, CTA 0 -> the other CTAs
     int* d_lpiv = nullptr;     // its row permutation
     int n_slaves_total = 0;          // slave dofs of every instance (multi-point constraints)
@@ -528,14 +529,8 @@ static int launch_large(StrutHandle* h, int mode, const DevInst* insts = nullptr
         int* lpiv = h->d_lpiv;
         void* args[] = {(void*)&insts, (void*)&A,  (void*)&ll,   (void*)&n_large, (void*)&mode,
                         (void*)&gb,    (void*)&wb, (void*)&lpan, (void*)&lpiv};
-        if (h->lfactor_wide)
-            CK(cudaLaunchCooperativeKernel((const void*)large_factor_kernel<kPanelWide, kLargeThreadsWide>,
-                                           dim3(h->lfactor_grid), dim3(kLargeThreadsWide), args, h->lfactor_smem,
-                                           h->stream));
-        else
-            CK(cudaLaunchCooperativeKernel((const void*)large_factor_kernel<kPanel, kLargeThreads>,
-                                           dim3(h->lfactor_grid), dim3(kLargeThreads), args, h->lfactor_smem,
-                                           h->stream));
+        CK(cudaLaunchCooperativeKernel(h->lfactor, dim3(h->lfactor_grid), dim3(h->lfactor_threads), args,
+                                       h->lfactor_smem, h->stream));
     }
     large_solve_kernel<<<h->n_large, kSolveThreads, large_solve_smem(h->max_large_n), h->stream>>>(insts, A, h->d_large_list, h->n_large, mode,
                                                                     h->d_wbuf, h->d_gb);
@@ -1307,9 +1302,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             for (int k = 0; k < I.n_att; ++k)
                 if (I.att_alg[k] != STRUT_ALGORITHM_NEWTON)
                     return bail(fail(STRUT_UNSUPPORTED, "ModifiedNewton on bands beyond shared memory is not implemented"));
-            const size_t fsm = bw > kLargeMaxBw ? large_factor_smem(kPanelWide, kLargeThreadsWide)
-                                                : large_factor_smem(kPanel, kLargeThreads);
-            if (fsm > 220 * 1024 || bw > kLargeMaxBwWide)
+            if (bw > kLargeMaxBwWide)
                 return bail(fail(STRUT_UNSUPPORTED, "band width too large for the blocked factorisation"));
             if (large_solve_smem(nf) > 220 * 1024)
                 return bail(fail(STRUT_UNSUPPORTED, "system too large for the band substitution"));
@@ -1321,7 +1314,6 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             h->large_list_h.push_back(inst);
             h->max_large_n = std::max(h->max_large_n, nf);
             h->max_large_bw = std::max(h->max_large_bw, bw);
-            h->lfactor_smem = std::max(h->lfactor_smem, fsm);
         } else {
             const size_t pad = (size_t)band_pad_rows(nf, bw, 6);
             h->inst_smem = std::max(h->inst_smem, ismem + pad * rw * sizeof(double));
@@ -1571,18 +1563,30 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             CK(cudaMemcpyAsync((char*)h->d_gb + offsetof(GridBarrier, limit), &polls, sizeof(int),
                                cudaMemcpyHostToDevice, h->stream));
         }
-        h->lfactor_wide = h->max_large_bw > kLargeMaxBw ? 1 : 0;
-        const void* fk = h->lfactor_wide ? (const void*)large_factor_kernel<kPanelWide, kLargeThreadsWide>
-                                         : (const void*)large_factor_kernel<kPanel, kLargeThreads>;
+        // one thread per panel row: the smallest variant that holds the widest band
+        const void* fk;
+        if (h->max_large_bw <= kLargeMaxBwNarrow) {
+            fk = (const void*)large_factor_kernel<kPanel, kLargeThreadsNarrow>;
+            h->lfactor_threads = kLargeThreadsNarrow;
+            h->lfactor_smem = large_factor_smem(kPanel, kLargeThreadsNarrow);
+        } else if (h->max_large_bw <= kLargeMaxBw) {
+            fk = (const void*)large_factor_kernel<kPanel, kLargeThreads>;
+            h->lfactor_threads = kLargeThreads;
+            h->lfactor_smem = large_factor_smem(kPanel, kLargeThreads);
+        } else {
+            fk = (const void*)large_factor_kernel<kPanelWide, kLargeThreadsWide>;
+            h->lfactor_threads = kLargeThreadsWide;
+            h->lfactor_smem = large_factor_smem(kPanelWide, kLargeThreadsWide);
+        }
+        h->lfactor = fk;
         CK(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->lfactor_smem));
         int per_sm = 0, n_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk, h->lfactor_wide ? kLargeThreadsWide : kLargeThreads,
-                                                         h->lfactor_smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk, h->lfactor_threads, h->lfactor_smem));
         CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
         if (per_sm < 1) return bail(fail(STRUT_UNSUPPORTED, "band factorisation kernel does not fit on an SM"));
         // one CTA per SM at most, all co-resident (cooperative launch), and no more than one
         // panel's trailing tiles can use
-        h->lfactor_grid = std::max(1, std::min(n_sm, large_factor_tiles(h->max_large_bw)));
+        h->lfactor_grid = std::max(1, std::min(n_sm, large_factor_tiles(h->max_large_bw, h->lfactor_threads)));
         h->default_factor_grid = h->lfactor_grid;
         h->max_factor_grid = n_sm * per_sm;
         CK(cudaFuncSetAttribute(large_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
