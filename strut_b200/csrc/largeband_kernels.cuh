@@ -322,7 +322,7 @@ __device__ __forceinline__ void warp_argmax_first(double& v, int& idx) {
 // publishes the panel; every CTA takes column tiles of the trailing block: loads them with the panel's row
 // permutation applied, solves the panel rows against the unit lower L11 on the warps (lane =
 // row), subtracts L21 U12 from the rows below entry by entry in column order (one thread per
-// row, the row's multipliers in registers); grid barrier.
+// row, the row's multipliers in registers) and counts itself off.
 template <int PANEL, int THREADS>
 __global__ void __launch_bounds__(THREADS) large_factor_kernel(
     const DevInst* __restrict__ insts, InstArrays A, const int* __restrict__ large_list,
