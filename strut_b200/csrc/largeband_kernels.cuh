@@ -44,10 +44,13 @@ constexpr int kSolveThreads = 1024;
 constexpr int kSolveAhead = 8;     // columns a lane of the substitution fetches a block ahead
 
 constexpr int kColTile = 16;       // trailing-update columns per tile
-// The variant for half bands up to 96 (15 nodes a floor): 128 threads, so every warp can look through
-// the whole column by itself and a panel column needs one barrier of four warps instead of two of
-// twelve; 8-column tiles, which double the CTAs of the trailing update.
+// Variants for half bands up to 96 and 160 (15 and 25 nodes a floor): 128 and 192 threads, so few warps that
+// every one looks through the whole column by itself and a panel column needs one barrier
+// instead of two of twelve warps; 8-column tiles, which double the CTAs of the trailing update.
+// Against 384 threads: n = 3000, half band 155 (8 steps) 87.4 -> 81.0 ms; n = 768, half band 101 12.6
+// -> 11.6 ms.  Every warp's look through the column grows with the square of the warps.
 constexpr int kLargeThreadsNarrow = 128;
+constexpr int kLargeThreadsMid = 192;
 constexpr int kColTileNarrow = 8;
 enum { LSTAT_OK = 0, LSTAT_SINGULAR = 2, LSTAT_CONVERGED = 7, LSTAT_IDLE = -1 };
 
@@ -273,7 +276,7 @@ __host__ __device__ constexpr int large_row_stride(int panel) {
     return panel + 1 > kColTile + 2 ? panel + 1 : kColTile + 2;
 }
 __host__ __device__ constexpr int large_col_tile(int threads) {
-    return threads == kLargeThreadsNarrow ? kColTileNarrow : kColTile;
+    return threads <= kLargeThreadsMid ? kColTileNarrow : kColTile;
 }
 __host__ __device__ inline size_t large_factor_smem(int panel, int threads) {
     return sizeof(double) * ((size_t)panel * (panel + 1) + (size_t)threads * large_row_stride(panel) + 4 * panel +
@@ -289,6 +292,7 @@ __host__ __device__ inline int large_factor_tiles(int bw, int threads) {
 
 // Largest half-band each variant takes: one thread per panel row.
 constexpr int kLargeMaxBwNarrow = kLargeThreadsNarrow - kPanel;
+constexpr int kLargeMaxBwMid = kLargeThreadsMid - kPanel;
 constexpr int kLargeMaxBw = kLargeThreads - kPanel;
 constexpr int kLargeMaxBwWide = kLargeThreadsWide - kPanelWide;
 
@@ -334,7 +338,7 @@ __global__ void __launch_bounds__(THREADS) large_factor_kernel(
     constexpr int kPs = PANEL + 1;     // row stride of L11
     constexpr int kRs = large_row_stride(PANEL);  // row stride of the panel rows and the slab
     constexpr int CT = large_col_tile(THREADS);
-    constexpr bool kNarrow = THREADS == kLargeThreadsNarrow;
+    constexpr bool kNarrow = THREADS <= kLargeThreadsMid;
     constexpr int kFly = kNarrow ? 8 : 4;  // loads in flight per thread
     constexpr int kSs = CT + 2;   // row stride of the slab (even: 16-byte rows)
     constexpr int kLd = THREADS;  // leading dimension of lpan

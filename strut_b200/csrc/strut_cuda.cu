@@ -1569,6 +1569,10 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             fk = (const void*)large_factor_kernel<kPanel, kLargeThreadsNarrow>;
             h->lfactor_threads = kLargeThreadsNarrow;
             h->lfactor_smem = large_factor_smem(kPanel, kLargeThreadsNarrow);
+        } else if (h->max_large_bw <= kLargeMaxBwMid) {
+            fk = (const void*)large_factor_kernel<kPanel, kLargeThreadsMid>;
+            h->lfactor_threads = kLargeThreadsMid;
+            h->lfactor_smem = large_factor_smem(kPanel, kLargeThreadsMid);
         } else if (h->max_large_bw <= kLargeMaxBw) {
             fk = (const void*)large_factor_kernel<kPanel, kLargeThreads>;
             h->lfactor_threads = kLargeThreads;
