@@ -1,4 +1,5 @@
-// Assembly of 3D instances as a kernel of its own: every band slot and every free dof's F_int sums
+// Assembly as a kernel of its own, for 3D instances and for every handle with a band in global memory
+// (whose kernels read the assembled slots): every band slot and every free dof's F_int sums
 // its list of element contributions (in assembly order, as the scatter of
 // stiffness_internal_frame2d.mojo:594-619 and its 3D counterpart add them up), times the collapse
 // coefficients of multi-point constraints.

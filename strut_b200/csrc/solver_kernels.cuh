@@ -33,8 +33,9 @@ struct InstArrays {
     const int* free_dof;  // absolute index of each free dof in u_full
     const double* Kinit;  // band, per instance at band_off
     const double* KinitT; // the same column by column (shared-memory bands; null without betaKInit)
-    const double* kband;  // 3D: K of every slot at band_off and F_int of every free dof, assembled by
-    const double* fsum;   // gather_kernel (null: the instance kernel gathers)
+    const double* kband;  // K of every slot at band_off and F_int of every free dof, assembled by
+    const double* fsum;   // gather_kernel (3D handles and those with a band in global memory; null: the
+                          // instance kernel gathers)
     const int8_t* efree;  // 2D without constraints: free dof of element dof b at 8 e + b, relative
                           // to the first free dof of the element (-1: none), and
     const int* efirst;    // that first free dof of element e in its instance

@@ -285,7 +285,7 @@ struct StrutHandle {
     std::vector<int> sec_off, sec_n;
     double* d_hist_sec = nullptr;
     long long ek_total = 0, ef_total = 0;
-    // 3D: assembled K and F_int (gather_kernel) and its grid
+    // 3D, and 2D with a band in global memory: assembled K and F_int (gather_kernel) and its grid
     double *d_kband = nullptr, *d_fsum = nullptr;
     int gather_slot_blocks = 0, gather_dof_blocks = 0;
     std::vector<DevShell> shells_h;  // linear shells of all instances
@@ -538,7 +538,8 @@ static int launch_large(StrutHandle* h, int mode, const DevInst* insts = nullptr
     return STRUT_OK;
 }
 
-// Assembly of a 3D handle's instances (gather_kernel) before the instance kernels that read it.
+// Assembly by gather_kernel before the instance kernels that read it: every instance of a 3D handle
+// and of one with bands in global memory (large_assemble_kernel reads nothing else).
 static dim3 gather_grid(const StrutHandle* h) {
     return dim3(h->gather_slot_blocks + h->gather_dof_blocks, h->n_inst);
 }
@@ -1523,7 +1524,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         std::vector<int> neg(h->n_inst, -1);
         if ((rc = upload(&h->d_fail_step, neg, al))) return bail(rc);
     }
-    if (h->ndf_all == 6) {
+    if (h->ndf_all == 6 || h->n_large > 0) {
         int slots = 0, dofs = 0;
         for (const DevInst& I : h->insts) {
             slots = std::max(slots, I.n * I.rw);
