@@ -20,6 +20,7 @@
 #pragma once
 
 #include "band_warp.cuh"
+#include "pivot_candidate.cuh"
 
 namespace strut {
 
@@ -54,31 +55,25 @@ __device__ __forceinline__ int band_lu_pivot(const double* Kb, int n, int bw, in
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
         const double* col = buf + 64 * (k & 1);
-        // pivot: the diagonal unless a row below beats it strictly, then the first largest
+        // pivot: the diagonal unless a row below beats it strictly, then the first largest.  A NaN on
+        // the diagonal is beaten by nothing (band LU), but once rows have been exchanged, as in the
+        // dense LU that Strut restarts with, the largest of the others takes its place.
         double v0 = lane < R ? col[lane] : 0.0;
         double v1 = lane + 32 < R ? col[lane + 32] : 0.0;
         const double akk = col[0];
         double piv = akk;
         int p = 0;
-        if (__any_sync(all, fabs(v0) > fabs(akk) || fabs(v1) > fabs(akk))) {
-            double bv = fabs(v0);
-            int br = lane;
-            if (fabs(v1) > bv) {
-                bv = fabs(v1);
-                br = lane + 32;
-            }
+        if (__any_sync(all, fabs(v0) > fabs(akk) || fabs(v1) > fabs(akk) || (nswap > 0 && akk != akk))) {
+            PivotCandidate best;
+            pivot_offer(best, fabs(v0), lane);
+            pivot_offer(best, fabs(v1), lane + 32);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ov = __shfl_xor_sync(all, bv, o);
-                const int orr = __shfl_xor_sync(all, br, o);
-                if (ov > bv || (ov == bv && orr < br)) {
-                    bv = ov;
-                    br = orr;
-                }
-            }
-            p = br;
+            for (int o = 16; o > 0; o >>= 1)
+                pivot_merge(best, __shfl_xor_sync(all, best.v, o), __shfl_xor_sync(all, best.row, o));
+            if (best.v <= 1.0e-14) return 2;  // the same on every lane of every warp
+            p = best.row;
             piv = col[p];
-            ++nswap;
+            nswap += p != 0;
         }
         if (fabs(piv) <= 1.0e-14) return 2;
         // the warp's columns: j0 .. j0 + 31
