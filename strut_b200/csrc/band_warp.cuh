@@ -142,7 +142,11 @@ __device__ __forceinline__ int band_lu_cta(double* B, int n, int bw, int rw, int
         else band_lu_rows<8, 1, 4, KEEP>(B, n, bw, rw, woff, rk, z, key);
     }
     __syncthreads();
-    return *key == kNoColumn ? 0 : *key & 1 ? 2 : 6;
+    if (*key == kNoColumn) return 0;
+    // a NaN diagonal gives way to nothing (the strict test): the loop's fmax took it for a small one, and
+    // what it computed is the elimination through it, NaN in every later pivot
+    const double d = B[(*key >> 1) * rw + bw];
+    return d != d ? 0 : *key & 1 ? 2 : 6;
 }
 
 // U x = w with one warp for bw <= kBackWarpMax, every row's sum in the reference's order (columns
