@@ -102,7 +102,10 @@ __device__ __forceinline__ void band_lu_rows(double* B, int n, int bw, int rw, i
             }
             swap = swap || fabs(f[u]) > d;
             big = big || fabs(f[u]) > dbig;
-            if (KEEP && lane == 0 && sf[u]) *const_cast<double*>(pf[u]) = q;
+            if constexpr (KEEP) {
+                if (u == 0) __syncwarp();  // every lane has read its multipliers' entries
+                if (lane == 0 && sf[u]) *const_cast<double*>(pf[u]) = q;
+            }
             pf[u] += sf[u];
         }
         const double rn = recip(a[0][0]);
