@@ -172,7 +172,8 @@ __device__ __forceinline__ void band_pivot_back(const double* U, double* Us, int
 }
 
 // Factor and solve: Kb (n x rw, shared memory) is replaced by U, w by L^-1 P w, x the solution.  U:
-// n x rw doubles of global memory.  The whole CTA of kPivotThreads threads; bw <= kPivotMaxBw.
+// n x rw doubles of global memory.  The whole CTA of kPivotThreads threads; bw <= kPivotMaxBw; regular
+// systems (quotient.cuh).
 // Returns 0 or 2 (singular); *swaps: interchanges made.
 __device__ __forceinline__ int band_pivot_solve(double* Kb, int n, int bw, int rw, double* w, double* x, double* U,
                                                 double* buf, int* swaps) {

@@ -129,8 +129,8 @@ __host__ __device__ inline int band_pad_rows(int n, int bw, int vectors) {
                ? bw : 0;
 }
 
-// band_lu_rows for half bands up to kLuRowsMax, by a CTA of kLuRowsThreads threads (all of them
-// call).  Returns 0 ok, 2 singular, 6 a row swap would be needed (the caller then starts again from
+// band_lu_rows for half bands up to kLuRowsMax and regular systems (quotient.cuh), by a CTA of
+// kLuRowsThreads threads (all of them call).  Returns 0 ok, 2 singular, 6 a row swap would be needed (the caller then starts again from
 // the assembled values), the same on all threads.  Four warps up to half band 31 (measured at 14 / 20: 226 / 273
 // cycles a step against 253 / 286 with eight), eight above.
 template <bool KEEP>
@@ -145,11 +145,7 @@ __device__ __forceinline__ int band_lu_cta(double* B, int n, int bw, int rw, int
         else band_lu_rows<8, 1, 4, KEEP>(B, n, bw, rw, woff, rk, z, key);
     }
     __syncthreads();
-    if (*key == kNoColumn) return 0;
-    // a NaN diagonal gives way to nothing (the strict test): the loop's fmax took it for a small one, and
-    // what it computed is the elimination through it, NaN in every later pivot
-    const double d = B[(*key >> 1) * rw + bw];
-    return d != d ? 0 : *key & 1 ? 2 : 6;
+    return *key == kNoColumn ? 0 : *key & 1 ? 2 : 6;
 }
 
 // U x = w with one warp for bw <= kBackWarpMax, every row's sum in the reference's order (columns
@@ -157,7 +153,8 @@ __device__ __forceinline__ int band_lu_cta(double* B, int n, int bw, int rw, int
 // unknown's first).  The unknowns a row needs and the next row's entries are in registers, so a row
 // costs its chain and a quotient (bw 20: 263 cycles; one lane with its operands in shared memory
 // took 810).  EXACT: bw == BW; else bw <= BW.  Slots of columns outside the matrix hold zeros.
-// rd: n doubles of scratch.
+// rd: n doubles of scratch.  Where an unknown is not finite, it and those before
+// it come out as NaN, x[0] with them (each takes up the one behind it, if only times zero).
 template <int BW, bool EXACT>
 __device__ __noinline__ void band_back_lu(const double* B, int n, int bw, int rw, const double* w, double* x,
                                           double* rd) {
@@ -209,7 +206,7 @@ __device__ __forceinline__ void band_back_lu_any(const double* B, int n, int bw,
 
 // L^T x = w with one warp for bw <= kBackWarpMax, column by column from the end (the reference's
 // order), a lane per row of the window, so that only a quotient and a shuffle separate one unknown
-// from the next.  rd: n doubles of scratch.
+// from the next.  rd: n doubles of scratch.  Not finite: as in band_back_lu.
 __device__ __noinline__ void band_back_chol(const double* B, int n, int bw, int rw, const double* w, double* x,
                                             double* rd) {
     constexpr unsigned all = 0xffffffffu;

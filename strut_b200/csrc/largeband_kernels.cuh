@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(THREADS) large_factor_kernel(
                         } else {
                             rare = __syncthreads_or(rare || fabs(offer) > dabs);
                         }
-                        double rpiv = recip(u[0]);  // beside the vote
+                        double rpiv = pivot_recip(u[0]);  // beside the vote
                         if (rare) {
                             // a NaN is no candidate: every thread has to find the same row
                             double pv = -1.0;
@@ -470,13 +470,13 @@ __global__ void __launch_bounds__(THREADS) large_factor_kernel(
                                 pivoted = 1;
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) u[q] = cb[q * THREADS + p];
-                                rpiv = recip(u[0]);
+                                rpiv = pivot_recip(u[0]);
                                 if (pos == c) pos = p;
                                 else if (pos == p) pos = c;
                             }
                         }
                         const bool below = pos > c;
-                        const double f = quot(a[0], u[0], rpiv);
+                        const double f = pivot_quot(a[0], u[0], rpiv);
                         a[0] = below ? f : a[0];
                         row[c] = a[0];
                         if (pos == c) s_perm[c] = r;

@@ -45,9 +45,14 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
     double* xs = w + n;
     double* fac = xs + n;
     // (columns before the first are never used, those behind the last have to be zeros)
+    int hi = 0;  // quotient.cuh: magnitude_hi of the largest entry
     if (!spd) {
 #pragma unroll 8
-        for (int t = tid; t < n * rw; t += nt) Kb[t] = band[t];
+        for (int t = tid; t < n * rw; t += nt) {
+            const double v = band[t];
+            Kb[t] = v;
+            hi = max(hi, magnitude_hi(v));
+        }
     } else {
 #pragma unroll 4
         for (int t = tid; t < n * (bw + 1); t += nt) {
@@ -55,20 +60,35 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
             Kb[i * rw + bw - (t - i * (bw + 1))] = band[t];
         }
     }
-    for (int i = tid; i < n; i += nt) R[i] = rhs[i];
-    __syncthreads();
+    for (int i = tid; i < n; i += nt) {
+        R[i] = rhs[i];
+        hi = max(hi, magnitude_hi(R[i]));
+    }
+    bool irregular = __syncthreads_or(hi >= kIrregularHi);
+    if (!spd && irregular) {
+        // what the caller left outside the matrix does not count
+        hi = 0;
+        for (int t = tid; t < n * rw; t += nt) {
+            const int j = t / rw + t % rw - bw;
+            if (j >= 0 && j < n) hi = max(hi, magnitude_hi(Kb[t]));
+        }
+        for (int i = tid; i < n; i += nt) hi = max(hi, magnitude_hi(R[i]));
+        irregular = __syncthreads_or(hi >= kIrregularHi);
+    }
+    const bool cta = !spd && bw <= pad && !irregular;
     if (!spd)
         for (int i = n - bw + tid; i < n; i += nt)
             for (int j = n; j <= i + bw; ++j) Kb[i * rw + bw + j - i] = 0.0;
+    if (cta) {
+        for (int i = tid; i < n; i += nt) w[i] = R[i];
+        for (int t = tid; t < pad * rw; t += nt) Kb[n * rw + t] = 0.0;
+    }
     __syncthreads();
     bool forward = false;  // w holds L^-1 rhs already
     int rc;
     if (spd) {
         rc = band_chol_smem(Kb, n, bw, rw, fac);
-    } else if (bw <= pad) {
-        for (int i = tid; i < n; i += nt) w[i] = R[i];
-        for (int t = tid; t < pad * rw; t += nt) Kb[n * rw + t] = 0.0;
-        __syncthreads();
+    } else if (cta) {
         rc = band_lu_cta<false>(Kb, n, bw, rw, (int)(w - Kb), s_rk, s_z, &s_key);
         forward = true;
     } else {

@@ -131,7 +131,7 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 }
 
 // Right-looking band LU without pivoting (Doolittle, unit-lower multipliers stored in place)
-// on the n x (2bw+1) band in shared memory, for half bands beyond kLuRowsMax (band_warp.cuh).  Step k computes the multiplier a_ik / a_kk of each
+// on the n x (2bw+1) band in shared memory, for half bands beyond kLuRowsMax (band_warp.cuh) and irregular systems (quotient.cuh).  Step k computes the multiplier a_ik / a_kk of each
 // row below the pivot once (fac, at least bw entries), checks the column for a row swap, then
 // updates the trailing block one warp per row.  Every entry receives the same single update
 // per step as in the reference's row loop.  Returns 0 ok, 2 singular, 6 a row swap would be
@@ -150,7 +150,7 @@ __device__ int band_lu_smem(double* B, int n, int bw, int rw, double* fac) {
             const double c = fabs(v);
             swap |= (c > aabs) ? 1 : 0;
             big |= (c > 1.0e-14) ? 1 : 0;
-            fac[t] = quot(v, akk, rkk);
+            fac[t] = full_quot(v, akk, rkk);
         }
         // pivot search of linear_solver_backend.mojo:640-657: an entry strictly larger than
         // the diagonal selects another row; the largest candidate decides singularity
@@ -187,7 +187,7 @@ __device__ int band_chol_smem(double* B, int n, int bw, int rw, double* fac) {
         const double lkk = sqrt(dkk), rkk = 1.0 / lkk;
         for (int t = tid; t < m; t += nt) {
             const int i = k + 1 + t;
-            fac[t] = quot(B[i * rw + (k - i + bw)], lkk, rkk);
+            fac[t] = full_quot(B[i * rw + (k - i + bw)], lkk, rkk);
         }
         __syncthreads();
         for (int r = warp; r < m; r += nw) {
@@ -207,8 +207,8 @@ __device__ int band_chol_smem(double* B, int n, int bw, int rw, double* fac) {
 // linear_solver_backend.mojo:735-770).  Forward: column-oriented, so row i receives
 // rhs_i - L_i,j0 w_j0 - L_i,j0+1 w_j0+1 - ... in increasing j, the order of the reference's row
 // loop.  Back: each row's sum in the reference's order, by band_back_lu for the bands it takes,
-// else by lane 0.  w may not alias rhs; rhs null: w holds
-// the forward sweep's result already.  rd: n doubles of scratch.
+// else (and again where that ended in a NaN, which may stand for an infinity) by lane 0.  w may not alias
+// rhs; rhs null: w holds the forward sweep's result already.  rd: n doubles of scratch.
 __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, int rw,
                                    const double* __restrict__ rhs, double* __restrict__ w,
                                    double* __restrict__ x, double* __restrict__ rd) {
@@ -227,7 +227,8 @@ __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, 
     }
     if (bw <= kBackWarpMax) {
         band_back_lu_any(B, n, bw, rw, w, x, rd);
-        return;
+        if (x[0] == x[0]) return;
+        __syncwarp();
     }
     if (lane == 0) {
         for (int i = n - 1; i >= 0; --i) {
@@ -262,7 +263,8 @@ __device__ void band_solve_chol_warp(const double* B, int n, int bw, int rw, con
     }
     if (bw <= kBackWarpMax) {
         band_back_chol(B, n, bw, rw, w, x, rd);
-        return;
+        if (x[0] == x[0]) return;
+        __syncwarp();
     }
     for (int i = lane; i < n; i += 32) x[i] = w[i];
     __syncwarp();
@@ -609,6 +611,8 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
     double* fac = du + n;
     const int f0 = I.f_off;
     int rc = 0;
+    int hi = 0;              // magnitude_hi of the largest entry of this thread's share of the system
+    bool irregular = false;  // some entry is not below 2^500 (quotient.cuh)
     // ModifiedNewton(Initial): the first iteration of the step freezes the tangent (the current
     // one, or K_init) and factors; later iterations reuse both (transient_nonlinear.mojo:
     // 2072-2085, 2236-2268, 2302-2335, 2421-2440)
@@ -617,9 +621,15 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
     const bool refresh = !modified || s_it == 0;
     double* Kfz = modified ? A.kfrz + I.band_off : nullptr;
     if (mode == INST_MODE_SOLVE_EXPORTED) {
-        for (int t = tid; t < n * rw; t += nt) Kb[t] = A.export_band[I.band_off + t];
-        for (int i = tid; i < n; i += nt) R[i] = A.rhs_in[f0 + i];
-        __syncthreads();
+        for (int t = tid; t < n * rw; t += nt) {
+            Kb[t] = A.export_band[I.band_off + t];
+            hi = max(hi, magnitude_hi(Kb[t]));
+        }
+        for (int i = tid; i < n; i += nt) {
+            R[i] = A.rhs_in[f0 + i];
+            hi = max(hi, magnitude_hi(R[i]));
+        }
+        irregular = __syncthreads_or(hi >= kIrregularHi);
     } else {
         if (mode == INST_MODE_NEWTON && tid == 0) {
             A.iters[inst] += 1;
@@ -744,6 +754,7 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
                     if (add_c) K[q] += I.a1 * C;
                     if (diag) K[q] += am;
                     if (in[q]) row[o0 + q] = K[q];
+                    hi = max(hi, magnitude_hi(K[q]));
                 }
             }
             double F;
@@ -758,9 +769,10 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
             const double ma = A.Mff[f0 + i] * w[i];
             R[i] = A.P_f[f0 + i] - F - 0.0 - cv - ma;
             A.R[f0 + i] = R[i];
+            hi = max(hi, magnitude_hi(R[i]));
             if (mode == INST_MODE_EXPORT) A.export_f[f0 + i] = F;
         }
-        __syncthreads();
+        irregular = __syncthreads_or(hi >= kIrregularHi);
         if (mode == INST_MODE_EXPORT) {
             for (int t = tid; t < n * rw; t += nt) A.export_band[I.band_off + t] = Kb[t];
             return;
@@ -843,7 +855,7 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
     bool forward = false;  // w holds L^-1 R already
     // an instance that has needed interchanges before goes straight to the pivoted factorisation,
     // which makes none where none is needed
-    const bool can_pivot = PIVOT && refresh && !modified && !I.spd && bw <= kPivotMaxBw;
+    const bool can_pivot = PIVOT && refresh && !modified && !I.spd && !irregular && bw <= kPivotMaxBw;
     bool pivoted = can_pivot && A.fallbacks && A.fallbacks[inst] > 0;
     int swaps = 0;
     if (pivoted) {
@@ -857,7 +869,7 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
         __syncthreads();
     } else if (I.spd) {
         rc = band_chol_smem(Kb, n, bw, rw, fac);
-    } else if (bw <= pad) {
+    } else if (bw <= pad && !irregular) {
         for (int i = tid; i < n; i += nt) w[i] = R[i];
         for (int t = tid; t < pad * rw; t += nt) Kb[n * rw + t] = 0.0;
         __syncthreads();
