@@ -800,7 +800,9 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     std::vector<double> sl_coef;
     std::vector<int8_t> efree8;  // 2D: free dofs of each element (InstArrays::efree)
     std::vector<int> efirst;
-    bool efree_ok = true;  // they fit eight bits relative to the first
+    // they fit eight bits relative to the first, and no element has one twice (ends that share a dof):
+    // the lanes of gather_rows each add to a slot of their own
+    bool efree_ok = true;
     bool any_kinit = false;
     bool any_mpc = false;
     for (int inst = 0; inst < num_instances; ++inst) any_mpc = any_mpc || models[inst].num_slaves > 0;
@@ -1067,6 +1069,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
                 for (int a = 0; a < 8; ++a) {
                     const int rel = a < 6 && fr[a] >= 0 ? fr[a] - lo : -1;
                     if (rel > 127) efree_ok = false;
+                    for (int b = 0; b < a && rel >= 0; ++b) efree_ok = efree_ok && fr[b] != fr[a];
                     efree8.push_back((int8_t)(rel > 127 ? -1 : rel));
                 }
             }
