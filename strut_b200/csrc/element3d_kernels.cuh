@@ -281,6 +281,7 @@ __device__ __forceinline__ bool invert5(double* a, double* inv) {
                 }
             }
         }
+        // (beyond 1e-40; an infinite pivot makes the row NaN with divisions too)
         const double piv = a[i * 5 + i], rp = 1.0 / piv;
 #pragma unroll
         for (int c = 0; c < 5; ++c) {

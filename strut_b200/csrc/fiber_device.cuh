@@ -155,6 +155,7 @@ __device__ __forceinline__ void concrete01_trial(const DevMat& m, const C1State&
 __device__ __forceinline__ void c2_compr_envlp(const DevMat& m, double strain, double& sig,
                                                double& tan) {
     const double fc = m.p[0], epsc0 = m.p[1], fcu = m.p[2], epscu = m.p[3];
+    // (quotients of strains between 0 and epscu by lengths of that order)
     if (strain >= epsc0) {
         const double rat = quot(strain, epsc0, m.k[C2K_REPSC0]);
         sig = fc * rat * (2.0 - rat);
@@ -197,13 +198,16 @@ struct C2Derived {
 __device__ __forceinline__ void concrete02_derive(const DevMat& m, const C2State& c, C2Derived& d) {
     double tmm;
     c2_compr_envlp(m, c.ecmin, d.sigmm, tmm);
+    // (an infinite ecmin: er is 0 or NaN and so ept NaN, and every strain is on the tension envelope, as it
+    // is with the infinite ept that divisions give)
     d.er = quot(d.sigmm - m.k[C2K_SIGMR], c.ecmin - m.k[C2K_EPSR]);
     d.ept = c.ecmin - quot(d.sigmm, d.er);
     d.epn = d.ept + c.dept;
     double sicn, tcn;
     c2_tens_envlp(m, c.dept, sicn, tcn);
     d.etn = m.k[C2K_EC0];
-    if (c.dept != 0.0) d.etn = quot(sicn, c.dept);
+    // (dept is infinite once a strain was; past the tension branch the quotient is 0 over any finite one)
+    if (c.dept != 0.0) d.etn = quot(sicn, below_infinity(c.dept));
 }
 
 // Stress and tangent for strain >= ecmin (unloading / reloading / tension branches).
@@ -347,6 +351,7 @@ __device__ __forceinline__ void steel02_branch(const DevMat& m, const S2State& c
 __device__ __forceinline__ void steel02_curve_of(const DevMat& m, const S2State& t, S2Curve& cv) {
     const double R0 = m.p[3], cR1 = m.p[4], cR2 = m.p[5];
     const double epsy = m.k[S2K_EPSY];
+    // (an infinite xi, or quot's NaN in its place: R is NaN)
     const double xi = fabs(quot(t.epspl - t.epss0, epsy, m.k[S2K_REPSY]));
     const double R = R0 * (1.0 - quot(cR1 * xi, cR2 + xi));
     cv.epsr = t.epsr;
@@ -362,7 +367,8 @@ __device__ __forceinline__ void steel02_curve_of(const DevMat& m, const S2State&
 __device__ __forceinline__ void steel02_curve_eval(const DevMat& m, const S2Curve& cv, double eps,
                                                    double& sig, double& tan) {
     const double b = m.p[2];
-    const double epsrat = quot(eps - cv.epsr, cv.denom, cv.rdenom);
+    // (eps is whatever a local iteration that diverges, or a caller's path, comes to)
+    const double epsrat = quot_or_inf(eps - cv.epsr, cv.denom, cv.rdenom);
     const double dum1 = 1.0 + pow(fabs(epsrat), cv.R);
     // far from the yield point |epsrat|^R vanishes beside 1, and 1^x is 1
     const double dum2 = dum1 == 1.0 ? 1.0 : pow(dum1, cv.invR);
