@@ -166,6 +166,9 @@ int strut_gpu_set_predictor(StrutHandle* h, StrutMlp* m, const float* x_mean, co
         (rc = up(d_xs, x_scale, (size_t)n_in * 4)) || (rc = up(d_ys, y_scale, (size_t)ndf * 4)) ||
         (rc = up(d_ag, ag.data(), ag.size() * 8)) || (rc = up(d_comp, comp.data(), comp.size() * 4)))
         return bail(rc);
+    // the caller's arrays (copied asynchronously if page-locked) are free again on return
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess)
+        return bail(fail(STRUT_CUDA_ERROR, "the predictor's arrays were not copied"));
     ps->P = PredDev{nn, ndf, n_in, h->n_free_total, h->n_inst, ag_len, d_nf, d_ni, d_nh, d_xm, d_xs, d_ys,
                     d_hist, d_ag, d_comp};
     h->pred = ps;
