@@ -82,6 +82,7 @@ extern "C" {
 int strut_gpu_set_predictor(StrutHandle* h, StrutMlp* m, const float* x_mean, const float* x_scale,
                             const float* y_scale) {
     if (!h) return fail(STRUT_BAD_ARG, "bad arguments");
+    h->graph_gen += 1;  // the graph holds the predictor's arrays, and a new one can have the old one's address
     if (h->pred) {
         pred_free(h->pred);
         h->pred = nullptr;

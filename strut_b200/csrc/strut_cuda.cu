@@ -348,7 +348,7 @@ struct StrutHandle {
     int* d_fail_step = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
-    const void* graph_keys[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    const void* graph_keys[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     double* d_rhs = nullptr;
     std::vector<long long> elem_fibers;  // fibers per element (all families)
     // node table of the learned predictor: nodes with a free dof, instance order then node order
@@ -361,8 +361,10 @@ struct StrutHandle {
     long long dense_total = 0;
     StrutTuning tune = {1, 0, 0, 0, {0, 0, 0, 0}};
     int default_factor_grid = 1;
-    int tune_gen = 0;       // bumped by strut_gpu_set_tuning (the graph bakes launch shapes in)
-    int graph_tune_gen = -1;
+    // bumped by strut_gpu_set_tuning and strut_gpu_set_predictor (the graph bakes launch shapes, arrays and
+    // the network in), and the value the graph was built at
+    int graph_gen = 0;
+    int built_gen = -1;
     ~StrutHandle();
     void release() {
         if (stream) cudaStreamSynchronize(stream);
@@ -751,16 +753,14 @@ static int build_graph(StrutHandle* h) {
     h->graph_keys[1] = h->d_hist_ef;
     h->graph_keys[2] = h->d_hist_iters;
     h->graph_keys[3] = h->d_ag;
-    h->graph_keys[5] = h->d_hist_sec;
-    h->graph_keys[4] = h->pred;
-    h->graph_tune_gen = h->tune_gen;
+    h->graph_keys[4] = h->d_hist_sec;
+    h->built_gen = h->graph_gen;
     return STRUT_OK;
 }
 
 static int ensure_graph(StrutHandle* h) {
-    if (h->gexec && h->graph_tune_gen == h->tune_gen && h->graph_keys[0] == h->d_hist_disp && h->graph_keys[1] == h->d_hist_ef &&
-        h->graph_keys[2] == h->d_hist_iters && h->graph_keys[3] == h->d_ag && h->graph_keys[4] == h->pred &&
-        h->graph_keys[5] == h->d_hist_sec)
+    if (h->gexec && h->built_gen == h->graph_gen && h->graph_keys[0] == h->d_hist_disp && h->graph_keys[1] == h->d_hist_ef &&
+        h->graph_keys[2] == h->d_hist_iters && h->graph_keys[3] == h->d_ag && h->graph_keys[4] == h->d_hist_sec)
         return STRUT_OK;
     return build_graph(h);
 }
@@ -1991,7 +1991,7 @@ int strut_gpu_set_tuning(StrutHandle* h, const StrutTuning* t) {
         return fail(STRUT_UNSUPPORTED, "the element kernel with that many threads does not fit on an SM");
     }
     h->lfactor_grid = d.factor_ctas > 0 ? std::min(d.factor_ctas, h->max_factor_grid) : h->default_factor_grid;
-    h->tune_gen += 1;
+    h->graph_gen += 1;
     return STRUT_OK;
 }
 

@@ -36,3 +36,29 @@ def test_page_locked_arrays_are_read_before_the_return(gpu_lib):
         got = PR.device_features(an)  # of step 0: no increments yet
     X, _ = PR.raw_features(m, np.zeros((1, m.num_free)))
     assert np.allclose(got, (X[:got.shape[0]] - mean) * scale, rtol=1e-6, atol=1e-6)
+
+
+def test_another_predictor_takes_the_place_of_the_first(gpu_lib):
+    """Runs after the change are those of an analysis whose step loop is built anew for the second network
+    (a change of launch shape that gives the same results makes it so)."""
+    def predictor(seed):
+        p = PR.LearnedPredictor(3, seed=seed)
+        p.y_scale = np.full(3, 1e-4 * (seed + 1), np.float32)
+        return p
+
+    first, second = predictor(0), predictor(3)
+    runs = []
+    for rebuild in (False, True):
+        with gpu_lib.Analysis([_model(60)], tuned=False) as an:
+            first.attach(an)
+            an.run(20)
+            second.attach(an)
+            if rebuild:
+                an.set_tuning(element_threads=224)
+            an.run(20)
+            runs.append((*an.history(0), PR.stats(an)))
+            PR.detach(an)
+            an.run(20)
+            runs[-1] += an.history(0)
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
