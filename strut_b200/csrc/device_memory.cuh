@@ -1,4 +1,4 @@
-// Device memory of the library's objects (included once, by strut_cuda.cu).
+// Device memory of the library's objects and shared memory of its kernels (included once, by strut_cuda.cu).
 //
 // Creating and destroying an analysis used to make some seventy cudaMalloc / cudaFree calls, each of
 // which maps or unmaps memory and can wait for the whole device: 4 to 40 ms a handle, with single
@@ -111,6 +111,19 @@ int upload(T** dptr, const std::vector<T>& h, Arena& a) {
 template <typename T>
 int dzeros(T** dptr, size_t n, Arena& a) {
     return a.take((void**)dptr, n * sizeof(T));
+}
+
+// Lets a kernel take all the dynamic shared memory that the device has beside its static.  The limit
+// belongs to the function, not to a handle: set to one handle's need, it was lowered by the next,
+// smaller handle, and the larger one's next launch or graph was refused.
+int allow_shared_memory(const void* kernel) {
+    int dev = 0, optin = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes fa;
+    CK(cudaFuncGetAttributes(&fa, kernel));
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    return STRUT_OK;
 }
 
 }  // namespace

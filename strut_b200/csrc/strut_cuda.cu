@@ -432,7 +432,7 @@ static dim3 elem_block(const StrutHandle* h) { return dim3(elem_threads_of(h)); 
 // Resident CTAs of the element kernel the handle's tuning selects (its persistent grid).
 static int elem_grid_of(StrutHandle* h) {
     int per_sm = 0, n_sm = 0;
-    CK(cudaFuncSetAttribute(elem_kernel_of(h), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->elem_smem));
+    TRY(allow_shared_memory((const void*)elem_kernel_of(h)));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, elem_kernel_of(h), (int)elem_block(h).x, h->elem_smem));
     CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
     if (per_sm < 1) return fail(STRUT_UNSUPPORTED, "element kernel does not fit on an SM");
@@ -1349,8 +1349,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     if (h->elem_smem > 200 * 1024) return bail(fail(STRUT_UNSUPPORTED, "element fiber history exceeds shared memory"));
     h->elem_smem = std::max<size_t>(h->elem_smem, 16);
     if ((rc = elem_grid_of(h)) != STRUT_OK) return bail(rc);
-    CK(cudaFuncSetAttribute(inst_kernel_of(h), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)std::max<size_t>(h->inst_smem, 16)));
+    if ((rc = allow_shared_memory((const void*)inst_kernel_of(h))) != STRUT_OK) return bail(rc);
     Arena& al = h->mem;
     // geometry and definitions
     DevMat* d_mats;
@@ -1587,7 +1586,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             h->lfactor_smem = large_factor_smem(kPanelWide, kLargeThreadsWide);
         }
         h->lfactor = fk;
-        CK(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->lfactor_smem));
+        if ((rc = allow_shared_memory(fk)) || (rc = allow_shared_memory((const void*)large_solve_kernel))) return bail(rc);
         int per_sm = 0, n_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk, h->lfactor_threads, h->lfactor_smem));
         CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
@@ -1597,8 +1596,6 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         h->lfactor_grid = std::max(1, std::min(n_sm, large_factor_tiles(h->max_large_bw, h->lfactor_threads)));
         h->default_factor_grid = h->lfactor_grid;
         h->max_factor_grid = n_sm * per_sm;
-        CK(cudaFuncSetAttribute(large_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)large_solve_smem(h->max_large_n)));
     }
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
@@ -2188,7 +2185,7 @@ static int fs_configure(StrutSectionBatch* b) {
     b->n_tiles = (b->n_inst + kFsTile - 1) / kFsTile;
     b->grid = 0;
     if (b->smem + 1024 > (size_t)optin) return STRUT_OK;
-    CK(cudaFuncSetAttribute(fiber_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
+    TRY(allow_shared_memory((const void*)fiber_stream_kernel));
     int resident = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fiber_stream_kernel, fs_threads(b->L), b->smem));
     if (resident < 1) return STRUT_OK;
