@@ -113,16 +113,16 @@ int dzeros(T** dptr, size_t n, Arena& a) {
     return a.take((void**)dptr, n * sizeof(T));
 }
 
-// Lets a kernel take all the dynamic shared memory that the device has beside its static.  The limit
-// belongs to the function, not to a handle: set to one handle's need, it was lowered by the next,
-// smaller handle, and the larger one's next launch or graph was refused.
-int allow_shared_memory(const void* kernel) {
-    int dev = 0, optin = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+// Lets a kernel take that much dynamic shared memory.  The limit belongs to the function, not to a handle, so
+// it is only ever raised: set to each handle's need, it was lowered by a smaller handle and a larger
+// one's next launch or graph was refused.
+std::mutex g_smem_mu;
+int raise_shared_memory(const void* kernel, size_t bytes) {
+    std::lock_guard<std::mutex> lock(g_smem_mu);
     cudaFuncAttributes fa;
     CK(cudaFuncGetAttributes(&fa, kernel));
-    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    if ((size_t)fa.maxDynamicSharedSizeBytes < bytes)
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return STRUT_OK;
 }
 

@@ -432,7 +432,7 @@ static dim3 elem_block(const StrutHandle* h) { return dim3(elem_threads_of(h)); 
 // Resident CTAs of the element kernel the handle's tuning selects (its persistent grid).
 static int elem_grid_of(StrutHandle* h) {
     int per_sm = 0, n_sm = 0;
-    TRY(allow_shared_memory((const void*)elem_kernel_of(h)));
+    TRY(raise_shared_memory((const void*)elem_kernel_of(h), h->elem_smem));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, elem_kernel_of(h), (int)elem_block(h).x, h->elem_smem));
     CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
     if (per_sm < 1) return fail(STRUT_UNSUPPORTED, "element kernel does not fit on an SM");
@@ -1349,7 +1349,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     if (h->elem_smem > 200 * 1024) return bail(fail(STRUT_UNSUPPORTED, "element fiber history exceeds shared memory"));
     h->elem_smem = std::max<size_t>(h->elem_smem, 16);
     if ((rc = elem_grid_of(h)) != STRUT_OK) return bail(rc);
-    if ((rc = allow_shared_memory((const void*)inst_kernel_of(h))) != STRUT_OK) return bail(rc);
+    if ((rc = raise_shared_memory((const void*)inst_kernel_of(h), h->inst_smem)) != STRUT_OK) return bail(rc);
     Arena& al = h->mem;
     // geometry and definitions
     DevMat* d_mats;
@@ -1586,7 +1586,9 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
             h->lfactor_smem = large_factor_smem(kPanelWide, kLargeThreadsWide);
         }
         h->lfactor = fk;
-        if ((rc = allow_shared_memory(fk)) || (rc = allow_shared_memory((const void*)large_solve_kernel))) return bail(rc);
+        if ((rc = raise_shared_memory(fk, h->lfactor_smem)) ||
+            (rc = raise_shared_memory((const void*)large_solve_kernel, large_solve_smem(h->max_large_n))))
+            return bail(rc);
         int per_sm = 0, n_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk, h->lfactor_threads, h->lfactor_smem));
         CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
@@ -2185,7 +2187,7 @@ static int fs_configure(StrutSectionBatch* b) {
     b->n_tiles = (b->n_inst + kFsTile - 1) / kFsTile;
     b->grid = 0;
     if (b->smem + 1024 > (size_t)optin) return STRUT_OK;
-    TRY(allow_shared_memory((const void*)fiber_stream_kernel));
+    TRY(raise_shared_memory((const void*)fiber_stream_kernel, b->smem));
     int resident = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fiber_stream_kernel, fs_threads(b->L), b->smem));
     if (resident < 1) return STRUT_OK;
