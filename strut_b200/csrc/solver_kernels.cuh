@@ -58,6 +58,7 @@ struct InstArrays {
     double* dense;        // per instance n x n scratch for the partial-pivot fallback
     int* piv;             // per free dof
     int* fallbacks;       // per instance count of dense fallbacks
+    int* pivots;          // whether a Newton iteration of the instance has needed interchanges (3D)
     ElemList el;          // elements of the instances still iterating
     // learned predictor: the step starts from the learned guess (dual 1), whose first iteration
     // checks it against the Newmark predictor's (u_base); rejected: per instance, the step went
@@ -853,10 +854,11 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
     double* D = A.dense + I.dense_off;
     int* piv = A.piv + f0;
     bool forward = false;  // w holds L^-1 R already
-    // an instance that has needed interchanges before goes straight to the pivoted factorisation,
-    // which makes none where none is needed
+    // an instance whose Newton iterations have needed interchanges goes straight to the pivoted factorisation,
+    // which makes none where none is needed.  (Its substitution adds a row up in another order, so a
+    // run's bits are its own only if other calls, strut_gpu_factor_solve, neither set nor follow this.)
     const bool can_pivot = PIVOT && refresh && !modified && !I.spd && !irregular && bw <= kPivotMaxBw;
-    bool pivoted = can_pivot && A.fallbacks && A.fallbacks[inst] > 0;
+    bool pivoted = can_pivot && mode == INST_MODE_NEWTON && A.pivots[inst] != 0;
     int swaps = 0;
     if (pivoted) {
     } else if (!refresh) {
@@ -896,7 +898,10 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
         for (int i = tid; i < n; i += nt) w[i] = R[i];
         __syncthreads();
         rc = band_pivot_solve(Kb, n, bw, rw, w, du, D, s_pbuf, &swaps);
-        if (tid == 0 && swaps > 0 && A.fallbacks) A.fallbacks[inst] += 1;
+        if (tid == 0 && swaps > 0) {
+            if (A.fallbacks) A.fallbacks[inst] += 1;
+            if (mode == INST_MODE_NEWTON) A.pivots[inst] = 1;
+        }
     }
     if (refresh && rc == 6) {
         // BandGeneral: a row swap would be needed, so the whole effective matrix is factored

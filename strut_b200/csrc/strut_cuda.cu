@@ -1442,6 +1442,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         (rc = dzeros(&h->d_elem_err, (size_t)h->n_elem, al)) ||
         (rc = dzeros(&h->d_counters, 8, al)) || (rc = dzeros(&A.dense, (size_t)h->dense_total, al)) ||
         (rc = dzeros(&A.piv, nF, al)) || (rc = dzeros(&A.fallbacks, (size_t)h->n_inst, al)) ||
+        (rc = dzeros(&A.pivots, (size_t)h->n_inst, al)) ||
         (rc = dzeros(&A.el.list[0], (size_t)h->n_elem, al)) || (rc = dzeros(&A.el.list[1], (size_t)h->n_elem, al)) ||
         (rc = dzeros(&A.el.count, 2, al)) || (rc = dzeros(&A.el.next, 2, al)) ||
         (rc = dzeros(&A.el.hard[0], (size_t)kFanCap, al)) || (rc = dzeros(&A.el.hard[1], (size_t)kFanCap, al)) ||
