@@ -83,19 +83,25 @@ __device__ __forceinline__ double gather_list(long long c0, long long c1, const 
     return K;
 }
 
-// grid: (blocks of 256 slots, then of 256 dofs; instances).  kband: band slots (band_off), fsum:
-// F_int of the free dofs (f_off).
+// A block's items: 256 band slots of an instance from `first`, or 256 free dofs from -1 - first.  Blocks
+// exist for the items there are, in one dimension, so neither the number of instances nor their
+// difference in size matters (as a grid of the largest instance's blocks by instances, 65,535 was the limit).
+struct GatherBlock {
+    int inst, first;
+};
+
+// kband: band slots (band_off), fsum: F_int of the free dofs (f_off).
 __global__ void __launch_bounds__(256) gather_kernel(const DevInst* __restrict__ insts, InstArrays A, int newton,
-                                                     int slot_blocks, double* __restrict__ kband,
-                                                     double* __restrict__ fsum) {
+                                                     const GatherBlock* __restrict__ blocks,
+                                                     double* __restrict__ kband, double* __restrict__ fsum) {
     __shared__ __align__(16) double2 buf[8][32];
-    const int inst = blockIdx.y, warp = threadIdx.x >> 5;
+    const GatherBlock G = blocks[blockIdx.x];
+    const int inst = G.inst, warp = threadIdx.x >> 5;
     if (newton && !A.active[inst]) return;
     const DevInst& I = insts[inst];
-    const bool slots = (int)blockIdx.x < slot_blocks;
+    const bool slots = G.first >= 0;
     const int n_items = slots ? I.n * I.rw : I.n;
-    const int t = (blockIdx.x - (slots ? 0 : slot_blocks)) * 256 + threadIdx.x;
-    if (t - (int)threadIdx.x >= n_items) return;
+    const int t = (slots ? G.first : -1 - G.first) + threadIdx.x;
     long long c0 = 0, c1 = 0;
     if (t < n_items) {
         if (slots) {

@@ -287,7 +287,8 @@ struct StrutHandle {
     long long ek_total = 0, ef_total = 0;
     // 3D, and 2D with a band in global memory: assembled K and F_int (gather_kernel) and its grid
     double *d_kband = nullptr, *d_fsum = nullptr;
-    int gather_slot_blocks = 0, gather_dof_blocks = 0;
+    GatherBlock* d_gather = nullptr;
+    int gather_blocks = 0;
     std::vector<DevShell> shells_h;  // linear shells of all instances
     DevShell* d_shells = nullptr;
     int n_shells = 0;
@@ -542,13 +543,10 @@ static int launch_large(StrutHandle* h, int mode, const DevInst* insts = nullptr
 
 // Assembly by gather_kernel before the instance kernels that read it: every instance of a 3D handle
 // and of one with bands in global memory (large_assemble_kernel reads nothing else).
-static dim3 gather_grid(const StrutHandle* h) {
-    return dim3(h->gather_slot_blocks + h->gather_dof_blocks, h->n_inst);
-}
 static int launch_gather(StrutHandle* h, const DevInst* insts, int mode) {
     if (!h->d_kband || mode == INST_MODE_SOLVE_EXPORTED) return STRUT_OK;
-    gather_kernel<<<gather_grid(h), 256, 0, h->stream>>>(insts, h->A, mode == INST_MODE_NEWTON ? 1 : 0,
-                                                         h->gather_slot_blocks, h->d_kband, h->d_fsum);
+    gather_kernel<<<h->gather_blocks, 256, 0, h->stream>>>(insts, h->A, mode == INST_MODE_NEWTON ? 1 : 0, h->d_gather,
+                                                           h->d_kband, h->d_fsum);
     CK(cudaGetLastError());
     return STRUT_OK;
 }
@@ -711,8 +709,8 @@ static int build_graph(StrutHandle* h) {
     }
     if (h->d_kband) {
         cudaGraphNode_t n_g;
-        TRY(add_kernel_node(&n_g, ibody, &n_after_el, 1, gather_kernel, gather_grid(h), dim3(256), 0,
-                            (const DevInst*)h->d_insts, A, 1, h->gather_slot_blocks, h->d_kband, h->d_fsum));
+        TRY(add_kernel_node(&n_g, ibody, &n_after_el, 1, gather_kernel, dim3(h->gather_blocks), dim3(256), 0,
+                            (const DevInst*)h->d_insts, A, 1, (const GatherBlock*)h->d_gather, h->d_kband, h->d_fsum));
         n_after_el = n_g;
     }
     TRY(add_kernel_node(&n_in, ibody, &n_after_el, 1, inst_kernel_of(h), dim3(h->n_inst), dim3(256),
@@ -1528,13 +1526,14 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
         if ((rc = upload(&h->d_fail_step, neg, al))) return bail(rc);
     }
     if (h->ndf_all == 6 || h->n_large > 0) {
-        int slots = 0, dofs = 0;
-        for (const DevInst& I : h->insts) {
-            slots = std::max(slots, I.n * I.rw);
-            dofs = std::max(dofs, I.n);
+        std::vector<GatherBlock> gb;
+        for (int i = 0; i < h->n_inst; ++i) {
+            const DevInst& I = h->insts[i];
+            for (int t = 0; t < I.n * I.rw; t += 256) gb.push_back({i, t});
+            for (int t = 0; t < I.n; t += 256) gb.push_back({i, -1 - t});
         }
-        h->gather_slot_blocks = (slots + 255) / 256;
-        h->gather_dof_blocks = (dofs + 255) / 256;
+        h->gather_blocks = (int)gb.size();
+        if ((rc = upload(&h->d_gather, gb, al))) return bail(rc);
         if ((rc = dzeros(&h->d_kband, (size_t)h->band_total, al)) || (rc = dzeros(&h->d_fsum, nF, al)))
             return bail(rc);
         A.kband = h->d_kband;
