@@ -1145,7 +1145,8 @@ __global__ void predictor_kernel(const DevInst* __restrict__ insts, InstArrays A
 }
 
 // Newmark update after convergence (transient_nonlinear.mojo:594-647), and the displacement records
-// (n_rec entries of rec_dof; none: 0).  Neither depends on the commit, which runs beside it.
+// (n_rec entries of rec_dof; none: 0).  Neither depends on the commit, which runs beside it (the record
+// pass of 3D elements, which can end an instance, comes before it).
 __global__ void post_step_kernel(const DevInst* __restrict__ insts, InstArrays A,
                                  const int* __restrict__ free_inst, int n_free_total,
                                  const int* __restrict__ rec_dof, int n_rec, double* __restrict__ rec_out,

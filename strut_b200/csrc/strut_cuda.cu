@@ -731,9 +731,12 @@ static int build_graph(StrutHandle* h) {
         n_after_commit = n_rp;
     }
     const int npost = std::max(nF, h->n_rec_total);
-    TRY(add_kernel_node(&n_post, body, &n_inner, 1, post_step_kernel, dim3((npost + tb - 1) / tb), dim3(tb), 0,
-                        (const DevInst*)h->d_insts, A, (const int*)h->d_free_inst, nF, (const int*)h->d_rec_dof,
-                        h->n_rec_total, h->d_hist_disp, (const DevCtl*)h->d_ctl));
+    // beside the commit, but after the 3D record pass: an element that fails there ends its instance, whose
+    // velocities and accelerations then stay as they are (as in the host-driven loop)
+    TRY(add_kernel_node(&n_post, body, h->n_rec3 > 0 ? &n_after_commit : &n_inner, 1, post_step_kernel,
+                        dim3((npost + tb - 1) / tb), dim3(tb), 0, (const DevInst*)h->d_insts, A,
+                        (const int*)h->d_free_inst, nF, (const int*)h->d_rec_dof, h->n_rec_total, h->d_hist_disp,
+                        (const DevCtl*)h->d_ctl));
     cudaGraphNode_t last = n_after_commit;
     if (h->n_sec_slots > 0) {
         cudaGraphNode_t n_sec;
