@@ -91,6 +91,8 @@ struct Arena {
         int here = 0;
         cudaGetDevice(&here);
         if (here != dev) cudaSetDevice(dev);
+        // an object on the legacy default stream is used on streams of its callers
+        if (!s) cudaDeviceSynchronize();
         for (void* b : blocks) cudaFreeAsync(b, s);
         if (here != dev) cudaSetDevice(here);
         blocks.clear();

@@ -94,10 +94,7 @@ struct StrutMlp {
     int* d_err = nullptr;
     long long adam_step = 0;
     Arena mem;  // on the legacy default stream
-    ~StrutMlp() {
-        cudaDeviceSynchronize();  // an analysis may have run the network on its own stream
-        mem.release();
-    }
+    ~StrutMlp() { mem.release(); }  // waits for the analyses that ran the network on their own streams
     int n_params() const { return n_in * kMlpH + kMlpH + kMlpH * kMlpH + kMlpH + kMlpH * n_out + n_out; }
     strut::MlpDev dev() const { return strut::MlpDev{d_w1t, d_w2t, d_w3t, d_b1, d_b2, d_b3}; }
     strut::MlpTrainDev train_dev() const { return strut::MlpTrainDev{dev(), d_w2, d_w3}; }

@@ -368,6 +368,9 @@ struct StrutHandle {
     int built_gen = -1;
     ~StrutHandle();
     void release() {
+        int here = 0;  // the device the caller has current, which need not be the handle's
+        cudaGetDevice(&here);
+        if (here != device) cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
         mem.release();
         for (void* p : {(void*)d_hist_disp, (void*)d_hist_ef, (void*)d_hist_iters, (void*)d_hist_sec, (void*)d_ag})
@@ -377,6 +380,7 @@ struct StrutHandle {
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (stream) cudaStreamDestroy(stream);
+        if (here != device) cudaSetDevice(here);
     }
 };
 
@@ -2249,7 +2253,6 @@ int strut_gpu_section_batch_create(const StrutUniMaterial* materials, int32_t nu
 
 int strut_gpu_section_batch_destroy(StrutSectionBatch* b) {
     if (!b) return STRUT_BAD_ARG;
-    cudaDeviceSynchronize();
     delete b;
     return STRUT_OK;
 }
