@@ -361,9 +361,10 @@ void* strut_gpu_stream(const StrutHandle* h);
  *                (at most 5 points).
  *   factor_ctas  CTAs of the cooperative wide-band factorisation (1 .. its resident limit;
  *                0: the default, as many as one panel has trailing tiles).
- *   element_threads  threads of an element CTA: 640 (one CTA per SM), 320 (default), 224 or 160
- *                (2D only): as many CTAs per SM as registers and shared memory allow, more
- *                elements in flight.
+ *   element_threads  threads of an element CTA: 640 (one CTA per SM), 320 (default, but 640 for
+ *                force-based elements of more than 960 fibers where 320 puts no more elements in
+ *                flight), 224 or 160 (2D only): as many CTAs per SM as registers and shared memory
+ *                allow, more elements in flight.
  * strut_gpu_set_tuning with t = NULL restores the defaults. */
 typedef struct StrutTuning {
     int32_t fan_out;

@@ -362,6 +362,7 @@ struct StrutHandle {
     long long dense_total = 0;
     StrutTuning tune = {1, 0, 0, 0, {0, 0, 0, 0}};
     int default_factor_grid = 1;
+    int default_elem_threads = kTeamThreads / 2;
     // bumped by strut_gpu_set_tuning and strut_gpu_set_predictor (the graph bakes launch shapes, arrays and
     // the network in), and the value the graph was built at
     int graph_gen = 0;
@@ -423,9 +424,16 @@ static bool elem_threads_ok(const StrutHandle* h, int t) {
 // the element kernel with 640 / 320 / 224 threads (us): one 3x3 frame 35.5 / 34.4 / 35.0, 8 frames (447
 // elements) 71 / 53 / 55, 128 frames (7,204) 766 / 452 / 469, 32 4-story 3D frames (5,120) 1,217 / 703
 // / 750, a 12-story 3D frame (780) 220 / 152 / 156.
+// It is 640 where that puts no fewer elements in flight (no more elements than SMs, or one CTA an SM with 320
+// too) and a force-based element has more than three fibers a thread of 320: its local iteration is then
+// the time, above all where it subdivides.  Runs of 148-fiber sections with 640 / 320 threads (ms): 3x3 frame
+// of 5, 7, 10 points at 1.5 g 7.1 / 6.9, 21.1 / 22.2, 65 / 76 (at 0.3 g 6.0 / 5.8, 6.2 / 6.3, 6.7 / 6.7);
+// 32 frames (1,771 elements) of 7, 10 points at 0.4 g 24.1 / 19.3, 106 / 123.  Displacement-based
+// elements evaluate their sections once: 10 points, 5.9 / 5.8.
+constexpr int kForceFibers320 = 960;
 static int elem_threads_of(const StrutHandle* h) {
     return h->tune.element_threads != 0 && elem_threads_ok(h, h->tune.element_threads) ? h->tune.element_threads
-                                                                                        : kTeamThreads / 2;
+                                                                                        : h->default_elem_threads;
 }
 static ElemKernel elem_kernel_of(const StrutHandle* h) {
     return h->ndf_all == 6 ? element_state_kernel<3> : element_state_kernel<2>;
@@ -443,6 +451,16 @@ static int elem_grid_of(StrutHandle* h) {
     if (per_sm < 1) return fail(STRUT_UNSUPPORTED, "element kernel does not fit on an SM");
     h->elem_grid = std::max(1, std::min(h->n_elem, per_sm * n_sm));
     return STRUT_OK;
+}
+// The default of elem_threads_of, and its grid.  force_fibers: fibers of the largest force-based element.
+static int default_elem_threads(StrutHandle* h, long long force_fibers) {
+    TRY(elem_grid_of(h));
+    if (force_fibers <= kForceFibers320) return STRUT_OK;
+    int n_sm = 0;
+    CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
+    if (h->elem_grid > n_sm) return STRUT_OK;
+    h->default_elem_threads = kTeamThreads;
+    return elem_grid_of(h);
 }
 static int commit_team_of(const StrutHandle* h) {
     // the commit kernel is launched with at most kTeamThreads threads: team x points
@@ -812,6 +830,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     bool any_mpc = false;
     for (int inst = 0; inst < num_instances; ++inst) any_mpc = any_mpc || models[inst].num_slaves > 0;
     long long c2_total = 0, s2_total = 0, s1_total = 0, c1_total = 0;
+    long long force_fibers = 0;  // of the largest force-based element
     std::vector<int> sec_base(num_instances);
     int u_off = 0, f_off = 0;
     long long band_off = 0;
@@ -1054,6 +1073,8 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
                                 8 * (size_t)((three_d ? 2 : 1) * ((n_tot + 1) & ~1) + 2 * E.nip * n_tot);
             h->elem_smem = std::max(h->elem_smem, smem);
             h->elem_fibers.push_back((long long)E.nip * (sd.n_s2 + sd.n_c2 + sd.n_s1 + sd.n_c1 + sd.n_el));
+            if (ed.type == STRUT_ELEM_FORCE_BEAM_COLUMN_2D || ed.type == STRUT_ELEM_FORCE_BEAM_COLUMN_3D)
+                force_fibers = std::max(force_fibers, h->elem_fibers.back());
             {
                 // committed history read once (Concrete02 / Steel01 5 doubles, Concrete01 6,
                 // Steel02 10 doubles + kon), element state read + written, k and f written,
@@ -1353,7 +1374,7 @@ int strut_gpu_create(const StrutModelDesc* models, int32_t num_instances, int32_
     h->dense_total = dense_off;
     if (h->elem_smem > 200 * 1024) return bail(fail(STRUT_UNSUPPORTED, "element fiber history exceeds shared memory"));
     h->elem_smem = std::max<size_t>(h->elem_smem, 16);
-    if ((rc = elem_grid_of(h)) != STRUT_OK) return bail(rc);
+    if ((rc = default_elem_threads(h, force_fibers)) != STRUT_OK) return bail(rc);
     if ((rc = raise_shared_memory((const void*)inst_kernel_of(h), h->inst_smem)) != STRUT_OK) return bail(rc);
     Arena& al = h->mem;
     // geometry and definitions
