@@ -6,7 +6,7 @@
 //
 // A 2D frame's system (36 to 216 unknowns, half band 11 to 20) is a chain of n dependent steps of a
 // few hundred operations, so the time is the latency of a step.  Measured for 216 unknowns of half
-// band 20 (cycles per unknown): factorisation 1,230 -> 261, back substitution 810 -> 263 (the sums of a row
+// band 20 (cycles per unknown): factorisation 1,230 -> 246, back substitution 810 -> 262 (the sums of a row
 // taken column by column instead, 123, rounded differently and were dropped: a batch of long records
 // is chaotic at the rounding level, and one record of 256 ended elsewhere).
 #pragma once
@@ -130,9 +130,9 @@ __host__ __device__ inline int band_pad_rows(int n, int bw, int vectors) {
 }
 
 // band_lu_rows for half bands up to kLuRowsMax and regular systems (quotient.cuh), by a CTA of
-// kLuRowsThreads threads (all of them call).  Returns 0 ok, 2 singular, 6 a row swap would be needed (the caller then starts again from
-// the assembled values), the same on all threads.  Four warps up to half band 31 (measured at 14 / 20: 226 / 273
-// cycles a step against 253 / 286 with eight), eight above.
+// kLuRowsThreads threads (all of them call).  Returns 0 ok, 2 singular, 6 a row swap would be needed (the
+// caller then starts again from the assembled values), the same on all threads.  Four warps up to half
+// band 31 (half band 14 / 20: 229 / 246 cycles a step, with eight warps 330 / 318), eight above.
 template <bool KEEP>
 __device__ __forceinline__ int band_lu_cta(double* B, int n, int bw, int rw, int woff, double* rk, double* z,
                                            int* key) {
@@ -151,7 +151,7 @@ __device__ __forceinline__ int band_lu_cta(double* B, int n, int bw, int rw, int
 // U x = w with one warp for bw <= kBackWarpMax, every row's sum in the reference's order (columns
 // upwards from the diagonal, so the chain of a row runs through all its bw products, the newest
 // unknown's first).  The unknowns a row needs and the next row's entries are in registers, so a row
-// costs its chain and a quotient (bw 20: 263 cycles; one lane with its operands in shared memory
+// costs its chain and a quotient (bw 20: 262 cycles; one lane with its operands in shared memory
 // took 810).  EXACT: bw == BW; else bw <= BW.  Slots of columns outside the matrix hold zeros.
 // rd: n doubles of scratch.  Where an unknown is not finite, it and those before
 // it come out as NaN, x[0] with them (each takes up the one behind it, if only times zero).

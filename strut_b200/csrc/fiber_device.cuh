@@ -288,9 +288,6 @@ struct S2Curve {
     double dsig;   // sigs0 - sigr
     double R, invR;
 };
-struct S2Derived {
-    S2Curve up, dn;  // strain increasing / decreasing
-};
 
 // Branch state after an increment in direction `up` (fiber2d.mojo:1103-1187): everything of
 // the trial state except eps, sig and tan.  Call only when the no-change test failed.
@@ -421,28 +418,6 @@ __device__ __forceinline__ void steel02_trial(const DevMat& m, const S2State& c,
     S2Curve cv;
     steel02_curve_of(m, t, cv);
     steel02_curve_eval(m, cv, eps, t.sig, t.tan);
-}
-
-__device__ __forceinline__ void steel02_derive(const DevMat& m, const S2State& c, S2Derived& d) {
-    S2State t;
-    steel02_branch(m, c, true, t);
-    steel02_curve_of(m, t, d.up);
-    steel02_branch(m, c, false, t);
-    steel02_curve_of(m, t, d.dn);
-}
-
-// Stress and tangent of steel02_trial, given the committed state's derived branches.
-__device__ __forceinline__ void steel02_sig_tan(const DevMat& m, const S2State& c,
-                                                const S2Derived& d, double trial_eps,
-                                                double& sig, double& tan) {
-    const double eps = steel02_strain(m, trial_eps);
-    const double deps = eps - c.eps;
-    if (steel02_no_change(c, deps)) {
-        tan = m.p[1];
-        sig = m.p[10];
-        return;
-    }
-    steel02_curve_eval(m, steel02_up(c, deps) ? d.up : d.dn, eps, sig, tan);
 }
 
 // Steel01 bilinear kinematic return map.
