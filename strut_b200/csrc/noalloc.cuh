@@ -20,6 +20,16 @@ constexpr size_t kNoAllocSmemMax = kBandSmemMax;  // band + 4 vectors in shared 
 static __device__ __align__(256) double g_noalloc_dense[kNoAllocMaxN * kNoAllocMaxN];  // 2 MiB
 static __device__ __align__(256) int g_noalloc_piv[kNoAllocMaxN];
 
+// As back_again, in the layout of band_solve_one_kernel.
+__device__ __noinline__ void one_back_again(double* smem, int n, int bw, int spd, const int& by_band) {
+    const int rw = 2 * bw + 1;
+    double* w = smem + (size_t)(n + (spd ? 0 : band_pad_rows(n, bw, 4))) * rw + n;
+    if (!by_band || bw > kBackWarpMax) return;
+    __syncthreads();
+    if (threadIdx.x < 32) band_back_divide(smem, n, bw, rw, spd, w, w + n);
+    __syncthreads();
+}
+
 // One CTA: load the band (BandGeneral n x (2bw+1) as stored; BandSPD n x (bw+1) with slot
 // row*(bw+1) + (row-col), expanded into the lower half of the general layout), factor, fall back
 // to the dense LU in `dense` / `piv` when a row swap is needed, solve, write x and *status
@@ -36,6 +46,7 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
     __shared__ int red_r[32];
     __shared__ double s_rk[2], s_z[2];  // band_lu_cta
     __shared__ int s_key;
+    __shared__ int s_by_band;  // solved with the band's factors
     const int tid = threadIdx.x, nt = blockDim.x;
     const int rw = 2 * bw + 1;
     double* Kb = smem_one;
@@ -111,6 +122,7 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
         if (tid == 0) *status = rc;
         return;
     }
+    if (tid == 0) s_by_band = !use_dense;
     __syncthreads();
     if (tid < 32) {
         if (use_dense)
@@ -121,6 +133,7 @@ __global__ void __launch_bounds__(256) band_solve_one_kernel(const double* __res
             band_solve_lu_warp(Kb, n, bw, rw, forward ? nullptr : R, w, xs, fac);
     }
     __syncthreads();
+    if (xs[0] != xs[0]) one_back_again(smem_one, n, bw, spd, s_by_band);
     for (int i = tid; i < n; i += nt) x[i] = xs[i];
     if (tid == 0) *status = 0;
 }

@@ -208,8 +208,8 @@ __device__ int band_chol_smem(double* B, int n, int bw, int rw, double* fac) {
 // linear_solver_backend.mojo:735-770).  Forward: column-oriented, so row i receives
 // rhs_i - L_i,j0 w_j0 - L_i,j0+1 w_j0+1 - ... in increasing j, the order of the reference's row
 // loop.  Back: each row's sum in the reference's order, by band_back_lu for the bands it takes,
-// else (and again where that ended in a NaN, which may stand for an infinity) by lane 0.  w may not alias
-// rhs; rhs null: w holds the forward sweep's result already.  rd: n doubles of scratch.
+// else by lane 0.  w may not alias rhs; rhs null: w holds the forward sweep's result already.  rd: n doubles
+// of scratch.  band_back_divide may follow.
 __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, int rw,
                                    const double* __restrict__ rhs, double* __restrict__ w,
                                    double* __restrict__ x, double* __restrict__ rd) {
@@ -228,8 +228,7 @@ __device__ void band_solve_lu_warp(const double* __restrict__ B, int n, int bw, 
     }
     if (bw <= kBackWarpMax) {
         band_back_lu_any(B, n, bw, rw, w, x, rd);
-        if (x[0] == x[0]) return;
-        __syncwarp();
+        return;
     }
     if (lane == 0) {
         for (int i = n - 1; i >= 0; --i) {
@@ -264,8 +263,7 @@ __device__ void band_solve_chol_warp(const double* B, int n, int bw, int rw, con
     }
     if (bw <= kBackWarpMax) {
         band_back_chol(B, n, bw, rw, w, x, rd);
-        if (x[0] == x[0]) return;
-        __syncwarp();
+        return;
     }
     for (int i = lane; i < n; i += 32) x[i] = w[i];
     __syncwarp();
@@ -277,6 +275,32 @@ __device__ void band_solve_chol_warp(const double* B, int n, int bw, int rw, con
         const int first = max(0, row - bw);
         for (int col = first + lane; col < row; col += 32) x[col] -= B[row * rw + (col - row + bw)] * xr;
         __syncwarp();
+    }
+}
+
+// The back substitution with divisions, one warp.  For bands of up to kBackWarpMax whose substitution ended in a
+// NaN, which may stand for an infinity (w as the solve left it).
+__device__ __forceinline__ void band_back_divide(const double* B, int n, int bw, int rw, bool spd, const double* w,
+                                                 double* x) {
+    const int lane = threadIdx.x & 31;
+    if (spd)
+        for (int i = lane; i < n; i += 32) x[i] = w[i];
+    __syncwarp();
+#pragma unroll 1
+    for (int i = n - 1; i >= 0; --i) {
+        if (lane == 0) {
+            double s = spd ? x[i] : w[i];
+            const int j1 = spd ? i : min(n - 1, i + bw);
+#pragma unroll 1
+            for (int j = i + 1; j <= j1; ++j) s -= B[i * rw + (j - i + bw)] * x[j];
+            x[i] = s / B[i * rw + bw];
+        }
+        __syncwarp();
+        if (spd) {
+            const double xi = x[i];
+            for (int j = max(0, i - bw) + lane; j < i; j += 32) x[j] -= B[i * rw + (j - i + bw)] * xi;
+            __syncwarp();
+        }
     }
 }
 
@@ -576,6 +600,19 @@ __device__ void dense_solve_warp(const double* D, const int* piv, int n, const d
 __device__ void newton_tail(const DevInst& I, InstArrays& A, int inst, const double* du,
                             const double* R, int* hrow, double* red, int* red_r);
 
+// band_back_divide in the layout of an instance's shared memory, by the whole CTA after the barrier behind the
+// solve.  A call with nothing but addresses in shared memory as its arguments: what it works with
+// would otherwise take registers from the factorisation's and the substitution's loops (3 us an
+// iteration of the 216-unknown frame).
+__device__ __noinline__ void back_again(const DevInst& I, double* smem, const int& by_band) {
+    const int n = I.n, bw = I.bw, rw = I.rw;
+    double* w = smem + (size_t)(n + band_pad_rows(n, bw, 6)) * rw + 2 * n;
+    if (!by_band || bw > kBackWarpMax) return;
+    __syncthreads();
+    if (threadIdx.x < 32) band_back_divide(smem, n, bw, rw, I.spd, w, w + n);
+    __syncthreads();
+}
+
 // PIVOT: the instance for 3D handles, whose systems with rigid diaphragms need row interchanges in
 // every factorisation; they run band_pivot_solve (band_pivot.cuh).  Its registers would keep two 2D
 // instances from sharing an SM, and a 2D frame's system needs an interchange once in some thousand
@@ -586,6 +623,7 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
     __shared__ DevInst I;
     __shared__ double red[32];
     __shared__ int red_r[32];
+    __shared__ int s_by_band;  // solved with the band's factors
     __shared__ int s_it;  // this instance's Newton iterations of the step so far
     __shared__ double s_rk[2], s_z[2];  // band_lu_cta
     __shared__ int s_key;
@@ -948,6 +986,7 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
         return;
     }
     // multipliers of the last column were written in the loop except column n-1 (none below)
+    if (tid == 0) s_by_band = !pivoted && !dense;
     __syncthreads();
     if (tid < 32) {
         if (pivoted)
@@ -960,6 +999,7 @@ __device__ __forceinline__ void instance_newton(const DevInst* __restrict__ inst
             band_solve_lu_warp(Kb, n, bw, rw, forward ? nullptr : R, w, du, fac);
     }
     __syncthreads();
+    if (du[0] != du[0]) back_again(I, smem_inst, s_by_band);
     if (mode == INST_MODE_SOLVE_EXPORTED) {
         for (int i = tid; i < n; i += nt) A.du[f0 + i] = du[i];
         return;
