@@ -48,8 +48,10 @@ int fail(int code, const std::string& msg) {
 #define CK(call)                                                                          \
     do {                                                                                  \
         cudaError_t e_ = (call);                                                          \
-        if (e_ != cudaSuccess)                                                            \
+        if (e_ != cudaSuccess) {                                                          \
+            cudaGetLastError(); /* reported here, and not again by the thread's next call */ \
             return fail(STRUT_CUDA_ERROR, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+        }                                                                                 \
     } while (0)
 
 inline int round4(int x) { return (x + 3) & ~3; }
