@@ -132,9 +132,10 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 }
 
 // Right-looking band LU without pivoting (Doolittle, unit-lower multipliers stored in place)
-// on the n x (2bw+1) band in shared memory, for half bands beyond kLuRowsMax (band_warp.cuh) and irregular systems (quotient.cuh).  Step k computes the multiplier a_ik / a_kk of each
-// row below the pivot once (fac, at least bw entries), checks the column for a row swap, then
-// updates the trailing block one warp per row.  Every entry receives the same single update
+// on the n x (2bw+1) band in shared memory, for half bands beyond kLuRowsMax (band_warp.cuh) and
+// irregular systems (quotient.cuh).  Step k computes the multiplier a_ik / a_kk of each row below the
+// pivot once (fac, at least bw entries), checks the column for a row swap, then updates the trailing
+// block one warp per row.  Every entry receives the same single update
 // per step as in the reference's row loop.  Returns 0 ok, 2 singular, 6 a row swap would be
 // needed (the caller then factors the assembled matrix densely with partial pivoting).
 __device__ int band_lu_smem(double* B, int n, int bw, int rw, double* fac) {

@@ -784,8 +784,8 @@ static int build_graph(StrutHandle* h) {
 }
 
 static int ensure_graph(StrutHandle* h) {
-    if (h->gexec && h->built_gen == h->graph_gen && h->graph_keys[0] == h->d_hist_disp && h->graph_keys[1] == h->d_hist_ef &&
-        h->graph_keys[2] == h->d_hist_iters && h->graph_keys[3] == h->d_ag && h->graph_keys[4] == h->d_hist_sec)
+    if (h->gexec && h->built_gen == h->graph_gen && h->graph_keys[0] == h->d_hist_disp &&
+        h->graph_keys[1] == h->d_hist_ef && h->graph_keys[2] == h->d_hist_iters && h->graph_keys[3] == h->d_ag && h->graph_keys[4] == h->d_hist_sec)
         return STRUT_OK;
     return build_graph(h);
 }
